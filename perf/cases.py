@@ -24,6 +24,7 @@ import math
 from types import SimpleNamespace
 
 import torch
+import torch.utils.checkpoint
 
 from multimodal_training_b200.config.model_configs import get_model_config
 from multimodal_training_b200.data.synthetic import Sample
@@ -277,6 +278,171 @@ def run(s):
     out = {"norm": norm, "param": o.flat_param, "exp_avg": o.exp_avg, "exp_avg_sq": o.exp_avg_sq}
     if o.master is not None:
         out["master"] = o.master
+    return out
+
+
+# --------------------------------------------------------------------------------------
+# The same pass in 64 bits: plain PyTorch on the weights, tables and inputs that prepare() makes
+# --------------------------------------------------------------------------------------
+F64 = torch.float64
+
+
+def _checkpointed(fn, *args):
+    return torch.utils.checkpoint.checkpoint(fn, *args, use_reentrant=False) if torch.is_grad_enabled() else fn(*args)
+
+
+def _norm64(x, w, eps):
+    return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + eps) * w
+
+
+def _rotate64(x, cos, sin):
+    """x [T, heads, dim]"""
+    a, b = x.chunk(2, dim=-1)
+    return x * cos[:, None] + torch.cat((-b, a), -1) * sin[:, None]
+
+
+def _softmax64(q, k, v, causal):
+    s = q @ k.transpose(-1, -2) / math.sqrt(q.shape[-1])
+    if causal:
+        s = s.masked_fill(torch.ones(s.shape[-2:], dtype=torch.bool, device=s.device).triu(1), -math.inf)
+    return s.softmax(-1) @ v
+
+
+def _attention64(q, k, v, cu, causal):
+    """q [T, heads, dim], k and v [T, kv heads, dim]; sequences of one length together, long ones head by head."""
+    rep, heads = q.shape[1] // k.shape[1], q.shape[1]
+    out = torch.zeros_like(q)
+    lengths: dict[int, list[int]] = {}
+    for a, b in zip(cu[:-1], cu[1:]):
+        if b > a:
+            lengths.setdefault(b - a, []).append(a)
+    for n, starts in lengths.items():
+        rows = torch.tensor(starts, device=q.device)[:, None] + torch.arange(n, device=q.device)
+        if n > 1024:
+            for r in rows:
+                out = out.index_copy(0, r, torch.stack([
+                    _checkpointed(_softmax64, q[r, h], k[r, h // rep], v[r, h // rep], causal)
+                    for h in range(heads)], 1))
+            continue
+        flat = rows.flatten()
+        qs, ks, vs = (t[flat].view(len(starts), n, t.shape[1], -1).transpose(1, 2) for t in (q, k, v))
+        ks, vs = (t.repeat_interleave(rep, 1) for t in (ks, vs))
+        out = out.index_copy(0, flat, _softmax64(qs, ks, vs, causal).transpose(1, 2).reshape(flat.numel(), heads, -1))
+    return out
+
+
+def _block64(x, w, cos, sin, cu, causal, heads, kv, eps):
+    T, d = x.shape[0], cos.shape[1]
+    bias = lambda y, b: y if b is None else y + b  # noqa: E731
+    qkv = bias(_norm64(x, w["n1"], eps) @ w["qkv"].T, w["qkv_b"]).view(T, -1, d)
+    rot = _rotate64(qkv[:, :heads + kv], cos, sin)
+    a = _attention64(rot[:, :heads], rot[:, heads:], qkv[:, heads + kv:], cu, causal)
+    x = x + bias(a.reshape(T, -1) @ w["o"].T, w["o_b"])
+    g, u = bias(_norm64(x, w["n2"], eps) @ w["gu"].T, w["gu_b"]).chunk(2, dim=-1)
+    return x + bias((torch.nn.functional.silu(g) * u) @ w["down"].T, w["down_b"])
+
+
+def _weights64(model, grad: bool) -> dict:
+    return {n: p.detach().to(F64).requires_grad_(grad) for n, p in model.named_parameters()}
+
+
+def _vision64(W, v, pixels, plan):
+    cos, sin = plan.cos_dev.to(F64), plan.sin_dev.to(F64)
+    x = pixels.to(F64) @ W["patch_embed_w"].T
+    for i in range(v.depth):
+        w = {a: W.get(f"blocks.{i}.{b}") for a, b in (
+            ("n1", "norm1_w"), ("qkv", "qkv_w"), ("qkv_b", "qkv_b"), ("o", "proj_w"), ("o_b", "proj_b"), ("n2", "norm2_w"),
+            ("gu", "gate_up_w"), ("gu_b", "gate_up_b"), ("down", "down_w"), ("down_b", "down_b"))}
+        cu = plan.full_cu if i in v.fullatt_block_indexes else plan.win_cu
+        x = _checkpointed(lambda t, w=w, cu=cu: _block64(t, w, cos, sin, cu, False, v.num_heads, v.num_heads,
+                                                         v.rms_norm_eps), x)
+    x = _norm64(x, W["ln_q_w"], v.rms_norm_eps).reshape(-1, v.hidden_size * v.merge_unit)
+    x = torch.nn.functional.gelu(x @ W["merger_fc1_w"].T + W["merger_fc1_b"])
+    return x @ W["merger_fc2_w"].T + W["merger_fc2_b"]
+
+
+def _text64(W, t, x, cos, sin, cu):
+    for i in range(t.num_hidden_layers):
+        w = {a: W.get(f"layers.{i}.{b}") for a, b in (
+            ("n1", "ln1_w"), ("qkv", "qkv_w"), ("qkv_b", "qkv_b"), ("o", "o_w"), ("o_b", ""), ("n2", "ln2_w"),
+            ("gu", "gate_up_w"), ("gu_b", ""), ("down", "down_w"), ("down_b", ""))}
+        x = _checkpointed(lambda y, w=w: _block64(y, w, cos, sin, cu, True, t.num_attention_heads,
+                                                  t.num_key_value_heads, t.rms_norm_eps), x)
+    return _norm64(x, W["norm_w"], t.rms_norm_eps), W.get("lm_head", W["embed_tokens"])
+
+
+def _text_loss64(W, t, s, merged):
+    x = W["embed_tokens"][s.ids].index_copy(0, s.rows, merged)
+    h, head = _text64(W, t, x, s.cos.to(F64), s.sin.to(F64), s.seq.host)
+    rows = (s.labels >= 0).nonzero().flatten()
+    return _checkpointed(lambda a, b: torch.nn.functional.cross_entropy(a @ b.T, s.labels[rows]), h[rows], head)
+
+
+def _flat64(opt, pieces: dict):
+    """The tensors of `pieces` (by parameter name) where the optimizer's flat buffers hold them, zeros between."""
+    out = torch.zeros(opt.total, dtype=F64, device=DEV)
+    for n, o in zip(opt.names, opt.offsets):
+        out[o:o + pieces[n].numel()] = pieces[n].detach().flatten()
+    return out
+
+
+def _adamw64(opt, p, g, m, v, step):
+    """Weights and moments after one update in 64 bits; the decayed parameters lie in front."""
+    b1, b2 = opt.betas
+    m, v = b1 * m + (1 - b1) * g, b2 * v + (1 - b2) * g * g
+    update = (m / (1 - b1 ** step)) / ((v / (1 - b2 ** step)).sqrt() + opt.eps)
+    update[:opt.n_decay] += opt.weight_decay * p[:opt.n_decay]
+    return p - opt.lr * update, m, v
+
+
+def exact(case: dict, seed: int):
+    if case["kind"] == "optimizer":
+        s = prepare(case, seed)
+        o = s.opt
+        norm = torch.sqrt(sum(c.to(F64).square().sum() for c in o.flat_grad.split(1 << 26)))
+        g = o.flat_grad.to(F64) * torch.clamp(1.0 / (norm + 1e-6), max=1.0)
+        p, m, v = _adamw64(o, (o.flat_param if o.master is None else o.master).to(F64), g, o.exp_avg.to(F64),
+                           o.exp_avg_sq.to(F64), o.step_count + 1)
+        out = {"norm": norm.reshape(1), "param": p, "exp_avg": m, "exp_avg_sq": v}
+        return out if o.master is None else {**out, "master": p}
+    if work(case)["flops"] > 1.5e14:       # over 20 seconds in 64 bits
+        return None
+    s, cfg = prepare(case, seed), _config(case)
+    v, t = cfg.vision, cfg.text
+    if s.kind in ("encode", "evaluate"):
+        with torch.no_grad():
+            if s.kind == "encode":
+                return {"merged": _vision64(_weights64(s.vision, False), v, s.pixels, s.plan)}
+            plan = _vision_plan(s.grids, cfg)
+            merged = _vision64(_weights64(s.model.visual, False), v,
+                               s.pixels.index_select(0, plan.local_patch_index.to(DEV)), plan)
+            merged = torch.empty_like(merged).index_copy(0, plan.local_merged_ids.to(DEV), merged)
+            W, ids = _weights64(s.model.language_model, False), s.ids[0]
+            x = W["embed_tokens"][ids].index_copy(0, (ids == cfg.image_token_id).nonzero().flatten(), merged)
+            pos, _ = s.model.get_rope_index(s.ids, s.grids)
+            cos, sin = mrope_cos_sin(pos[:, 0], t.head_dim, t.rope_theta, t.mrope_section)
+            h, head = _text64(W, t, x, cos.to(DEV, F64), sin.to(DEV, F64), [0, ids.numel()])
+            return {"logits": h @ head.T}
+    out = {}
+    if s.kind in ("vision", "train"):
+        Wv = _weights64(s.vision, True)
+        merged = _vision64(Wv, v, s.pixels, s.plan)
+    if s.kind in ("text", "train"):
+        Wt = _weights64(s.text, True)
+        leaf = (s.merged.to(F64) if s.kind == "text" else merged.detach()).requires_grad_(True)
+        loss = _text_loss64(Wt, t, s, leaf)
+        loss.backward()
+        text_grad = _flat64(s.text_opt, {n: w.grad for n, w in Wt.items()})
+    if s.kind == "text":
+        return {"loss": loss.detach(), "vision_grad": leaf.grad, "grad": text_grad}
+    merged.backward(s.grad.to(F64) if s.kind == "vision" else leaf.grad)
+    vision_grad = _flat64(s.vision_opt, {n: w.grad for n, w in Wv.items()})
+    if s.kind == "vision":
+        return {"merged": merged.detach(), "grad": vision_grad}
+    out = {"loss": loss.detach(), "vision_grad": vision_grad, "text_grad": text_grad}
+    for name, opt, grad in (("vision", s.vision_opt, vision_grad), ("text", s.text_opt, text_grad)):
+        p = opt.flat_param.to(F64)
+        out[name] = _adamw64(opt, p, grad, torch.zeros_like(p), torch.zeros_like(p), 1)[0]
     return out
 
 
