@@ -67,29 +67,6 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int X2 = 64;
-  // the two items of this CTA: heads fastest, so both usually share the query rows (and, with GQA, K and V)
-  int q0[2], head[2], kv_lo[2], n_tiles[2], xq[2], xk[2], xv[2];
-#pragma unroll
-  for (int w = 0; w < 2; ++w) {
-    // causal: the last query tiles see the most KV tiles, so they are started first (longest work first)
-    const int cta = p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
-    const int item = cta * 2 + w;
-    n_tiles[w] = 0;
-    q0[w] = head[w] = kv_lo[w] = xq[w] = xk[w] = xv[w] = 0;
-    if (item < n_items) {
-      head[w] = item % p.n_q;
-      q0[w] = (item / p.n_q) * BQ;
-      const int kv_head = head[w] / (p.n_q / p.n_kv);
-      const int q_last = min(q0[w] + BQ, p.T) - 1;
-      kv_lo[w] = p.seq_lo[q0[w]];
-      const int kv_hi = p.causal ? min(p.seq_hi[q_last], q_last + 1) : p.seq_hi[q_last];
-      n_tiles[w] = (kv_hi - kv_lo[w] + BKV - 1) / BKV;
-      xq[w] = head[w] * DIM;
-      xk[w] = (p.n_q + kv_head) * DIM;
-      xv[w] = (p.n_q + p.n_kv + kv_head) * DIM;
-    }
-  }
-  const int max_tiles = max(n_tiles[0], n_tiles[1]);
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm);
@@ -113,6 +90,30 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_sync();
+  // the two items of this CTA: heads fastest, so both usually share the query rows (and, with GQA, K and V)
+  int q0[2], head[2], kv_lo[2], n_tiles[2], xq[2], xk[2], xv[2];
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    // causal: the last query tiles see the most KV tiles, so they are started first (longest work first)
+    const int cta = p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+    const int item = cta * 2 + w;
+    n_tiles[w] = 0;
+    q0[w] = head[w] = kv_lo[w] = xq[w] = xk[w] = xv[w] = 0;
+    if (item < n_items) {
+      head[w] = item % p.n_q;
+      q0[w] = (item / p.n_q) * BQ;
+      const int kv_head = head[w] / (p.n_q / p.n_kv);
+      const int q_last = min(q0[w] + BQ, p.T) - 1;
+      kv_lo[w] = p.seq_lo[q0[w]];
+      const int kv_hi = p.causal ? min(p.seq_hi[q_last], q_last + 1) : p.seq_hi[q_last];
+      n_tiles[w] = (kv_hi - kv_lo[w] + BKV - 1) / BKV;
+      xq[w] = head[w] * DIM;
+      xk[w] = (p.n_q + kv_head) * DIM;
+      xv[w] = (p.n_q + p.n_kv + kv_head) * DIM;
+    }
+  }
+  const int max_tiles = max(n_tiles[0], n_tiles[1]);
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
@@ -334,7 +335,8 @@ int launch_fwd2(const CUtensorMap& tm, const AttnParams& p, cudaStream_t st) {
     attr = true;
   }
   const int n_items = ((p.T + BQ - 1) / BQ) * p.n_q;
-  attn_fwd2_kernel<DIM><<<(n_items + 1) / 2, kFwd2Threads, kFwdSmem, st>>>(tm, p, n_items);
+  launch_dependent(attn_fwd2_kernel<DIM>, (n_items + 1) / 2, kFwd2Threads, kFwdSmem, st,
+                     tm, p, n_items);
   return (int)cudaGetLastError();
 }
 

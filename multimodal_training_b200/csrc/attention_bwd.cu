@@ -21,6 +21,7 @@ using namespace attn;
 // ----------------------------------------------------------------------------------------------
 __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
                                   float* __restrict__ delta, int T, int n_q, int dim) {
+  grid_dependency_sync();
   const long w = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= (long)T * n_q) return;
@@ -67,6 +68,7 @@ MMT_DEVICE void store_chunk(uint8_t* tile, int row, int c, const uint32_t (&pk)[
 // dK / dV of a GQA group = sum of its q heads' fp32 partials, in head order (deterministic), rounded once.
 __global__ void attn_group_reduce_kernel(const float* __restrict__ ws_dk, const float* __restrict__ ws_dv,
                                          __nv_bfloat16* __restrict__ dqkv, int T, int n_q, int n_kv, int dim, long ld) {
+  grid_dependency_sync();
   const int group = n_q / n_kv;
   const int per_row = n_kv * dim / 4;                 // float4 items per token and tensor
   const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -134,18 +136,6 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kv0 = blockIdx.x * BKV;
-  const bool split = p.ws_dk != nullptr;
-  const int full_group = p.n_q / p.n_kv;
-  const int kv_head = split ? (int)blockIdx.y / full_group : (int)blockIdx.y;
-  const int head0 = split ? (int)blockIdx.y : kv_head * full_group;
-  const int group = split ? 1 : full_group;
-  const int kv_last = min(kv0 + BKV, p.T) - 1;
-  const int q_lo = p.causal ? kv0 : p.seq_lo[kv0];
-  const int q_hi = p.seq_hi[kv_last];
-  const int n_qb = (q_hi - q_lo + BQ2 - 1) / BQ2;
-  const int n_iter = n_qb * group;
-  const int xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm_kv);
@@ -171,6 +161,19 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_sync();
+  const int kv0 = blockIdx.x * BKV;
+  const bool split = p.ws_dk != nullptr;
+  const int full_group = p.n_q / p.n_kv;
+  const int kv_head = split ? (int)blockIdx.y / full_group : (int)blockIdx.y;
+  const int head0 = split ? (int)blockIdx.y : kv_head * full_group;
+  const int group = split ? 1 : full_group;
+  const int kv_last = min(kv0 + BKV, p.T) - 1;
+  const int q_lo = p.causal ? kv0 : p.seq_lo[kv0];
+  const int q_hi = p.seq_hi[kv_last];
+  const int n_qb = (q_hi - q_lo + BQ2 - 1) / BQ2;
+  const int n_iter = n_qb * group;
+  const int xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
   const uint32_t t_dv = tmem_base + 256, t_dk = tmem_base + 384;
 
   if (warp == 8) {
@@ -404,15 +407,6 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // causal: the last query tiles see the most KV blocks and are started first
-  const int q0 = (p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x) * BQ;
-  const int head = blockIdx.y;
-  const int kv_head = head / (p.n_q / p.n_kv);
-  const int q_last = min(q0 + BQ, p.T) - 1;
-  const int kv_lo = p.seq_lo[q0];
-  const int kv_hi = p.causal ? min(p.seq_hi[q_last], q_last + 1) : p.seq_hi[q_last];
-  const int n_iter = (kv_hi - kv_lo + BQ2 - 1) / BQ2;
-  const int xq = head * DIM, xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm_q);
@@ -438,6 +432,16 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_sync();
+  // causal: the last query tiles see the most KV blocks and are started first
+  const int q0 = (p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x) * BQ;
+  const int head = blockIdx.y;
+  const int kv_head = head / (p.n_q / p.n_kv);
+  const int q_last = min(q0 + BQ, p.T) - 1;
+  const int kv_lo = p.seq_lo[q0];
+  const int kv_hi = p.causal ? min(p.seq_hi[q_last], q_last + 1) : p.seq_hi[q_last];
+  const int n_iter = (kv_hi - kv_lo + BQ2 - 1) / BQ2;
+  const int xq = head * DIM, xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
   const uint32_t t_dq = tmem_base + 256;
 
   if (warp == 8) {
@@ -611,13 +615,16 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap&
     attr = true;
   }
   const int tiles = (p.T + BQ - 1) / BQ;
-  attn_bwd_dkdv2_kernel<DIM><<<dim3(tiles, p.ws_dk ? p.n_q : p.n_kv), kBwd2Threads, kBwd2Smem, st>>>(tq, tq64, tdo64, p);
+  launch_dependent(attn_bwd_dkdv2_kernel<DIM>, dim3(tiles, p.ws_dk ? p.n_q : p.n_kv), kBwd2Threads, kBwd2Smem, st,
+                     tq, tq64, tdo64, p);
   if (p.ws_dk) {
     const long items = (long)p.T * (p.n_kv * DIM / 4) * 2;
-    attn_group_reduce_kernel<<<(unsigned)((items + 255) / 256), 256, 0, st>>>(p.ws_dk, p.ws_dv, p.dqkv, p.T, p.n_q,
+    launch_dependent(attn_group_reduce_kernel, (unsigned)((items + 255) / 256), 256, 0, st,
+                     p.ws_dk, p.ws_dv, p.dqkv, p.T, p.n_q,
                                                                              p.n_kv, DIM, p.ld);
   }
-  attn_bwd_dq2_kernel<DIM><<<dim3(tiles, p.n_q), kBwd2Threads, kDq2Smem, st>>>(tq, tdo, tq64, p);
+  launch_dependent(attn_bwd_dq2_kernel<DIM>, dim3(tiles, p.n_q), kBwd2Threads, kDq2Smem, st,
+                     tq, tdo, tq64, p);
   return (int)cudaGetLastError();
 }
 
@@ -637,7 +644,8 @@ extern "C" int mmt_attn_bwd(const void* qkv, const void* out, const void* dout, 
     const long warps = T * n_q;
     const int threads = 256;
     const long blocks = (warps * 32 + threads - 1) / threads;
-    attn_delta_kernel<<<(unsigned)blocks, threads, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(out),
+    launch_dependent(attn_delta_kernel, (unsigned)blocks, threads, 0, st,
+                     reinterpret_cast<const __nv_bfloat16*>(out),
                                                            reinterpret_cast<const __nv_bfloat16*>(dout), delta,
                                                            (int)T, n_q, dim);
   }

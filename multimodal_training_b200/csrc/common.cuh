@@ -57,6 +57,21 @@ MMT_DEVICE uint64_t mmt_globaltimer() {
 #endif
 
 // ---------------------------------------------------------------------------
+// Programmatic dependent launch (host side: launch_dependent in runtime.h)
+// ---------------------------------------------------------------------------
+// First statement of a kernel that may be launched while its predecessor in the stream still runs: returns when every
+// earlier grid has finished and its writes are visible, then lets the next kernel's CTAs take the SM resources that
+// this grid leaves free.  Nothing in front of it may touch global memory (barrier set-up, tensor-memory allocation and
+// descriptor prefetches may); EVERY thread block has to execute it, so that "this grid has finished" implies the same
+// of all grids before it.
+MMT_DEVICE void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+MMT_DEVICE void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+MMT_DEVICE void grid_dependency_sync() {
+  grid_dependency_wait();
+  grid_dependents_launch();
+}
+
+// ---------------------------------------------------------------------------
 // Shared-memory address helpers
 // ---------------------------------------------------------------------------
 MMT_DEVICE uint32_t smem_u32(const void* p) {

@@ -82,6 +82,7 @@ constexpr int kNormVec = 4;  // up to 8192 columns
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_fwd_kernel(const bf16* __restrict__ x,
                                                                   const bf16* __restrict__ w, bf16* __restrict__ y,
                                                                   float* __restrict__ rstd_out, int cols, float eps) {
+  grid_dependency_sync();
   __shared__ float red[32];
   const long row = blockIdx.x;
   const bf16* xr = x + row * cols;
@@ -131,6 +132,7 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_fwd_warp_kernel(const bf
                                                                        bf16* __restrict__ y,
                                                                        float* __restrict__ rstd_out, long rows,
                                                                        int cols, float eps) {
+  grid_dependency_sync();
   const int lane = threadIdx.x & 31;
   const long row = (long)blockIdx.x * (kNormThreads / 32) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -182,6 +184,7 @@ __global__ void __launch_bounds__(kNormThreads, VEC <= 2 ? 2 : 1) rmsnorm_bwd_ke
                                                                      bf16* __restrict__ dx,
                                                                      float* __restrict__ dw_partial, int rows, int cols,
                                                                      const bf16* __restrict__ extra) {
+  grid_dependency_sync();
   constexpr int kWarps = kNormThreads / 32;
   __shared__ float red[2][R][kWarps];
   const int nvec = cols >> 3;
@@ -275,6 +278,7 @@ __global__ void __launch_bounds__(kNormThreads, VEC <= 2 ? 2 : 1) rmsnorm_bwd_ke
 // lanes with independent loads and combined in a fixed order, so the result does not depend on scheduling.
 __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, bf16* __restrict__ out,
                                                               int parts, int cols, int accumulate) {
+  grid_dependency_sync();
   __shared__ float red[8][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
@@ -300,6 +304,7 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
 // ----------------------------------------------------------------------------
 __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                             long tokens, int heads, int dim, long row_stride, float sign) {
+  grid_dependency_sync();
   const int half = dim >> 1;
   const int pairs_per_head = half >> 1;  // two adjacent columns per thread
   const long total = tokens * heads * pairs_per_head;
@@ -339,6 +344,7 @@ __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cos_
 // matching eight of the high half (needs dim / 2 to be a multiple of 8).
 __global__ void __launch_bounds__(256, 4) rope_vec8_kernel(bf16* __restrict__ x, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                  long tokens, int heads, int dim, long row_stride, float sign) {
+  grid_dependency_sync();
   const int half = dim >> 1;
   const int vecs = half >> 3;
   const long total = tokens * heads * vecs;
@@ -383,6 +389,7 @@ __global__ void __launch_bounds__(256, 4) rope_vec8_kernel(bf16* __restrict__ x,
 // SwiGLU on a fused [rows, 2*inter] gate|up buffer.
 // ----------------------------------------------------------------------------
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long rows, int inter) {
+  grid_dependency_sync();
   const int nvec = inter >> 3;
   const long total = rows * nvec;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -399,6 +406,7 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
 
 __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu,
                                   long rows, int inter) {
+  grid_dependency_sync();
   const int nvec = inter >> 3;
   const long total = rows * nvec;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -421,6 +429,7 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __r
 }
 
 __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long n8) {
+  grid_dependency_sync();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
     float v[8];
     load8(x + i * 8, v);
@@ -431,6 +440,7 @@ __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y
 }
 __global__ void gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, bf16* __restrict__ dx,
                                 long n8) {
+  grid_dependency_sync();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
     float v[8], d[8];
     load8(x + i * 8, v);
@@ -443,6 +453,7 @@ __global__ void gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restr
 
 // y = a + b (bf16), used for residual adds outside GEMM epilogues.
 __global__ void add_kernel(const bf16* __restrict__ a, const bf16* __restrict__ b, bf16* __restrict__ y, long n8) {
+  grid_dependency_sync();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
     float u[8], v[8];
     load8(a + i * 8, u);
@@ -459,6 +470,7 @@ __global__ void add_kernel(const bf16* __restrict__ a, const bf16* __restrict__ 
 // ----------------------------------------------------------------------------
 __global__ void gather_rows_kernel(const bf16* __restrict__ src, const long* __restrict__ idx, bf16* __restrict__ dst,
                                    long rows, int cols, long lo, long hi, long src_ld, long dst_ld) {
+  grid_dependency_sync();
   const long r = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -474,6 +486,7 @@ __global__ void gather_rows_kernel(const bf16* __restrict__ src, const long* __r
 // dst[idx[r]] = src[r]   (add == 0)   or   dst[idx[r]] += src[r]  (add == 1, bf16x2 atomics)
 __global__ void scatter_rows_kernel(const bf16* __restrict__ src, const long* __restrict__ idx, bf16* __restrict__ dst,
                                     long rows, int cols, long lo, long hi, long src_ld, long dst_ld, int add) {
+  grid_dependency_sync();
   const long r = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -495,6 +508,7 @@ __global__ void scatter_rows_kernel(const bf16* __restrict__ src, const long* __
 // ----------------------------------------------------------------------------
 __global__ void colsum_partial_kernel(const bf16* __restrict__ x, float* __restrict__ partial, long rows, int cols,
                                       long ld) {
+  grid_dependency_sync();
   // blockDim = (32 column-vectors, 8 row lanes); grid = (ceil(cols/256), row splits)
   __shared__ float red[8][32][8];
   const int cv = blockIdx.x * 32 + threadIdx.x;
@@ -533,6 +547,7 @@ __global__ void __launch_bounds__(kCeThreads) ce_stats_kernel(const bf16* __rest
                                                              const long* __restrict__ labels, float* __restrict__ omax,
                                                              float* __restrict__ osum, float* __restrict__ otgt, int V,
                                                              long ld, long vocab_lo) {
+  grid_dependency_sync();
   __shared__ float red[32];
   const long row = blockIdx.x;
   const bf16* l = logits + row * ld;
@@ -567,6 +582,7 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* __restrict__ 
                                                             const float* __restrict__ gsum,
                                                             const float* __restrict__ scale_ptr, int V, long ld,
                                                             long vocab_lo) {
+  grid_dependency_sync();
   const long row = blockIdx.x;
   bf16* l = logits + row * ld;
   const int nvec = V >> 3;
@@ -598,6 +614,7 @@ __global__ void adamw_kernel(bf16* __restrict__ p, const bf16* __restrict__ g, f
                              float* __restrict__ m, float* __restrict__ v, long n, long n_decay, float lr, float b1,
                              float b2, float eps, float wd, float bc1, float bc2,
                              const float* __restrict__ gscale_ptr) {
+  grid_dependency_sync();
   const float gs = gscale_ptr ? *gscale_ptr : 1.f;
   const long n8 = n >> 3;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
@@ -637,6 +654,7 @@ __global__ void adamw_kernel(bf16* __restrict__ p, const bf16* __restrict__ g, f
 __global__ void adamw_bf16_kernel(bf16* __restrict__ p, const bf16* __restrict__ g, bf16* __restrict__ m,
                                   bf16* __restrict__ v, long n, long n_decay, float lr, float b1, float b2, float eps,
                                   float wd, float bc1, float bc2, const float* __restrict__ gscale_ptr) {
+  grid_dependency_sync();
   const float gs = gscale_ptr ? *gscale_ptr : 1.f;
   const long n8 = n >> 3;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
@@ -663,6 +681,7 @@ __global__ void adamw_bf16_kernel(bf16* __restrict__ p, const bf16* __restrict__
 
 // out[0] += sum(x^2)   (fp32 atomic; caller zeroes out)
 __global__ void sumsq_kernel(const bf16* __restrict__ x, long n8, float* __restrict__ out) {
+  grid_dependency_sync();
   __shared__ float red[32];
   float s = 0.f;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
@@ -678,6 +697,7 @@ __global__ void sumsq_kernel(const bf16* __restrict__ x, long n8, float* __restr
 // coef = min(1, max_norm / (sqrt(normsq) + 1e-6)) * extra
 __global__ void clip_coef_kernel(const float* __restrict__ normsq, float max_norm, float extra,
                                  float* __restrict__ coef) {
+  grid_dependency_sync();
   const float n = sqrtf(*normsq);
   float c = max_norm > 0.f ? fminf(1.f, max_norm / (n + 1e-6f)) : 1.f;
   *coef = c * extra;
@@ -704,11 +724,14 @@ int mmt_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long row
   const int vpl = (cols / 8 + 31) / 32;
   const unsigned grid8 = (unsigned)((rows + kNormThreads / 32 - 1) / (kNormThreads / 32));
   if (vpl <= 8) {
-    rmsnorm_fwd_warp_kernel<8><<<grid8, kNormThreads, 0, ST(stream)>>>(CBF(x), CBF(w), BF(y), rstd, rows, cols, eps);
+    launch_dependent(rmsnorm_fwd_warp_kernel<8>, grid8, kNormThreads, 0, ST(stream),
+                     CBF(x), CBF(w), BF(y), rstd, rows, cols, eps);
   } else if (vpl <= 16) {
-    rmsnorm_fwd_warp_kernel<16><<<grid8, kNormThreads, 0, ST(stream)>>>(CBF(x), CBF(w), BF(y), rstd, rows, cols, eps);
+    launch_dependent(rmsnorm_fwd_warp_kernel<16>, grid8, kNormThreads, 0, ST(stream),
+                     CBF(x), CBF(w), BF(y), rstd, rows, cols, eps);
   } else {
-    rmsnorm_fwd_kernel<<<(unsigned)rows, kNormThreads, 0, ST(stream)>>>(CBF(x), CBF(w), BF(y), rstd, cols, eps);
+    launch_dependent(rmsnorm_fwd_kernel, (unsigned)rows, kNormThreads, 0, ST(stream),
+                     CBF(x), CBF(w), BF(y), rstd, cols, eps);
   }
   return (int)cudaGetLastError();
 }
@@ -721,7 +744,8 @@ int mmt_rmsnorm_bwd_parts(long rows) {
 
 static void launch_reduce_partials(const float* scratch, void* out, int parts, int cols, int accumulate,
                                    void* stream) {
-  reduce_partials_kernel<<<(cols + 31) / 32, dim3(32, 8), 0, ST(stream)>>>(scratch, BF(out), parts, cols, accumulate);
+  launch_dependent(reduce_partials_kernel, (cols + 31) / 32, dim3(32, 8), 0, ST(stream),
+                     scratch, BF(out), parts, cols, accumulate);
 }
 
 // Launches the backward kernel on at most `max_parts` CTAs; returns the number of partial rows it wrote.
@@ -733,7 +757,7 @@ static int launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
   if (grid > max_parts) grid = max_parts;
   if (grid < 1) grid = 1;
 #define MMT_NORM_BWD(V, RR)                                                                                        \
-  rmsnorm_bwd_kernel<V, RR><<<(unsigned)grid, kNormThreads, 0, ST(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), \
+  launch_dependent(rmsnorm_bwd_kernel<V, RR>, (unsigned)grid, kNormThreads, 0, ST(stream), CBF(dy), CBF(x), CBF(w), rstd, BF(dx), \
                                                                              scratch, (int)rows, cols, CBF(extra))
   switch (vec) {
     case 1: MMT_NORM_BWD(1, 4); break;
@@ -779,11 +803,12 @@ int mmt_rope(void* x, const float* cos_t, const float* sin_t, long tokens, int h
                          reinterpret_cast<uintptr_t>(sin_t)) & 15) == 0;
   if (dim % 16 == 0 && row_stride % 8 == 0 && aligned) {
     const long work8 = tokens * heads * (dim / 16);
-    rope_vec8_kernel<<<grid_for(work8, 256, mmt_sm_count() * 8), 256, 0, ST(stream)>>>(
-        BF(x), cos_t, sin_t, tokens, heads, dim, row_stride, backward ? -1.f : 1.f);
+    launch_dependent(rope_vec8_kernel, grid_for(work8, 256, mmt_sm_count() * 8), 256, 0, ST(stream),
+                     BF(x), cos_t, sin_t, tokens, heads, dim, row_stride, backward ? -1.f : 1.f);
     return (int)cudaGetLastError();
   }
-  rope_kernel<<<grid_for(work, 256, mmt_sm_count() * 8), 256, 0, ST(stream)>>>(BF(x), cos_t, sin_t, tokens, heads, dim,
+  launch_dependent(rope_kernel, grid_for(work, 256, mmt_sm_count() * 8), 256, 0, ST(stream),
+                     BF(x), cos_t, sin_t, tokens, heads, dim,
                                                                               row_stride, backward ? -1.f : 1.f);
   return (int)cudaGetLastError();
 }
@@ -792,33 +817,38 @@ int mmt_swiglu_fwd(const void* gu, void* out, long rows, int inter, void* stream
   if (inter % 8) return -2;
   const long work = rows * (inter / 8);
   if (work == 0) return 0;
-  swiglu_fwd_kernel<<<grid_for(work, 256, mmt_sm_count() * 8), 256, 0, ST(stream)>>>(CBF(gu), BF(out), rows, inter);
+  launch_dependent(swiglu_fwd_kernel, grid_for(work, 256, mmt_sm_count() * 8), 256, 0, ST(stream),
+                     CBF(gu), BF(out), rows, inter);
   return (int)cudaGetLastError();
 }
 int mmt_swiglu_bwd(const void* dout, const void* gu, void* dgu, long rows, int inter, void* stream) {
   if (inter % 8) return -2;
   const long work = rows * (inter / 8);
   if (work == 0) return 0;
-  swiglu_bwd_kernel<<<grid_for(work, 256, mmt_sm_count() * 8), 256, 0, ST(stream)>>>(CBF(dout), CBF(gu), BF(dgu), rows,
+  launch_dependent(swiglu_bwd_kernel, grid_for(work, 256, mmt_sm_count() * 8), 256, 0, ST(stream),
+                     CBF(dout), CBF(gu), BF(dgu), rows,
                                                                                     inter);
   return (int)cudaGetLastError();
 }
 int mmt_gelu_fwd(const void* x, void* y, long n, void* stream) {
   if (n % 8) return -2;
   if (n == 0) return 0;
-  gelu_fwd_kernel<<<grid_for(n / 8, 256, mmt_sm_count() * 8), 256, 0, ST(stream)>>>(CBF(x), BF(y), n / 8);
+  launch_dependent(gelu_fwd_kernel, grid_for(n / 8, 256, mmt_sm_count() * 8), 256, 0, ST(stream),
+                     CBF(x), BF(y), n / 8);
   return (int)cudaGetLastError();
 }
 int mmt_gelu_bwd(const void* dy, const void* x, void* dx, long n, void* stream) {
   if (n % 8) return -2;
   if (n == 0) return 0;
-  gelu_bwd_kernel<<<grid_for(n / 8, 256, mmt_sm_count() * 8), 256, 0, ST(stream)>>>(CBF(dy), CBF(x), BF(dx), n / 8);
+  launch_dependent(gelu_bwd_kernel, grid_for(n / 8, 256, mmt_sm_count() * 8), 256, 0, ST(stream),
+                     CBF(dy), CBF(x), BF(dx), n / 8);
   return (int)cudaGetLastError();
 }
 int mmt_add(const void* a, const void* b, void* y, long n, void* stream) {
   if (n % 8) return -2;
   if (n == 0) return 0;
-  add_kernel<<<grid_for(n / 8, 256, mmt_sm_count() * 8), 256, 0, ST(stream)>>>(CBF(a), CBF(b), BF(y), n / 8);
+  launch_dependent(add_kernel, grid_for(n / 8, 256, mmt_sm_count() * 8), 256, 0, ST(stream),
+                     CBF(a), CBF(b), BF(y), n / 8);
   return (int)cudaGetLastError();
 }
 
@@ -826,7 +856,8 @@ int mmt_gather_rows(const void* src, const long* idx, void* dst, long rows, int 
                     long dst_ld, void* stream) {
   if (cols % 8 || src_ld % 8 || dst_ld % 8) return -2;
   if (rows == 0) return 0;
-  gather_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, ST(stream)>>>(CBF(src), idx, BF(dst), rows, cols, lo, hi,
+  launch_dependent(gather_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, ST(stream),
+                     CBF(src), idx, BF(dst), rows, cols, lo, hi,
                                                                         src_ld, dst_ld);
   return (int)cudaGetLastError();
 }
@@ -834,7 +865,8 @@ int mmt_scatter_rows(const void* src, const long* idx, void* dst, long rows, int
                      long dst_ld, int add, void* stream) {
   if (cols % 8 || src_ld % 8 || dst_ld % 8) return -2;
   if (rows == 0) return 0;
-  scatter_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, ST(stream)>>>(CBF(src), idx, BF(dst), rows, cols, lo, hi,
+  launch_dependent(scatter_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, ST(stream),
+                     CBF(src), idx, BF(dst), rows, cols, lo, hi,
                                                                          src_ld, dst_ld, add);
   return (int)cudaGetLastError();
 }
@@ -849,7 +881,8 @@ int mmt_colsum(const void* x, void* out, float* scratch, long rows, int cols, lo
   if (cols % 8 || ld % 8) return -2;
   const int parts = mmt_colsum_parts(rows);
   dim3 grid((cols + 255) / 256, parts), block(32, 8);
-  colsum_partial_kernel<<<grid, block, 0, ST(stream)>>>(CBF(x), scratch, rows, cols, ld);
+  launch_dependent(colsum_partial_kernel, grid, block, 0, ST(stream),
+                     CBF(x), scratch, rows, cols, ld);
   launch_reduce_partials(scratch, out, parts, cols, accumulate, stream);
   return (int)cudaGetLastError();
 }
@@ -858,7 +891,8 @@ int mmt_ce_stats(const void* logits, const long* labels, float* omax, float* osu
                  long ld, long vocab_lo, void* stream) {
   if (V % 8 || ld % 8) return -2;
   if (rows == 0) return 0;
-  ce_stats_kernel<<<(unsigned)rows, kCeThreads, 0, ST(stream)>>>(CBF(logits), labels, omax, osum, otgt, V, ld,
+  launch_dependent(ce_stats_kernel, (unsigned)rows, kCeThreads, 0, ST(stream),
+                     CBF(logits), labels, omax, osum, otgt, V, ld,
                                                                 vocab_lo);
   return (int)cudaGetLastError();
 }
@@ -866,7 +900,8 @@ int mmt_ce_grad(void* logits, const long* labels, const float* gmax, const float
                 long rows, int V, long ld, long vocab_lo, void* stream) {
   if (V % 8 || ld % 8) return -2;
   if (rows == 0) return 0;
-  ce_grad_kernel<<<(unsigned)rows, kCeThreads, 0, ST(stream)>>>(BF(logits), labels, gmax, gsum, scale_ptr, V, ld,
+  launch_dependent(ce_grad_kernel, (unsigned)rows, kCeThreads, 0, ST(stream),
+                     BF(logits), labels, gmax, gsum, scale_ptr, V, ld,
                                                                vocab_lo);
   return (int)cudaGetLastError();
 }
@@ -876,8 +911,8 @@ int mmt_adamw(void* p, const void* g, float* master, float* m, float* v, long n,
   if (n % 8) return -2;
   if (n == 0) return 0;
   const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-  adamw_kernel<<<grid_for(n / 8, 256, mmt_sm_count() * 16), 256, 0, ST(stream)>>>(
-      BF(p), CBF(g), master, m, v, n, n_decay, lr, b1, b2, eps, wd, bc1, bc2, gscale_ptr);
+  launch_dependent(adamw_kernel, grid_for(n / 8, 256, mmt_sm_count() * 16), 256, 0, ST(stream),
+                     BF(p), CBF(g), master, m, v, n, n_decay, lr, b1, b2, eps, wd, bc1, bc2, gscale_ptr);
   return (int)cudaGetLastError();
 }
 
@@ -887,19 +922,21 @@ int mmt_adamw_bf16(void* p, const void* g, void* m, void* v, long n, long n_deca
   if (n % 8) return -2;
   if (n == 0) return 0;
   const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-  adamw_bf16_kernel<<<grid_for(n / 8, 256, mmt_sm_count() * 16), 256, 0, ST(stream)>>>(
-      BF(p), CBF(g), BF(m), BF(v), n, n_decay, lr, b1, b2, eps, wd, bc1, bc2, gscale_ptr);
+  launch_dependent(adamw_bf16_kernel, grid_for(n / 8, 256, mmt_sm_count() * 16), 256, 0, ST(stream),
+                     BF(p), CBF(g), BF(m), BF(v), n, n_decay, lr, b1, b2, eps, wd, bc1, bc2, gscale_ptr);
   return (int)cudaGetLastError();
 }
 
 int mmt_sumsq(const void* x, long n, float* out, void* stream) {
   if (n % 8) return -2;
   if (n == 0) return 0;
-  sumsq_kernel<<<grid_for(n / 8, 256, mmt_sm_count() * 8), 256, 0, ST(stream)>>>(CBF(x), n / 8, out);
+  launch_dependent(sumsq_kernel, grid_for(n / 8, 256, mmt_sm_count() * 8), 256, 0, ST(stream),
+                     CBF(x), n / 8, out);
   return (int)cudaGetLastError();
 }
 int mmt_clip_coef(const float* normsq, float max_norm, float extra, float* coef, void* stream) {
-  clip_coef_kernel<<<1, 1, 0, ST(stream)>>>(normsq, max_norm, extra, coef);
+  launch_dependent(clip_coef_kernel, 1, 1, 0, ST(stream),
+                     normsq, max_norm, extra, coef);
   return (int)cudaGetLastError();
 }
 

@@ -67,6 +67,7 @@ struct GemmParams {
   int group_m, tiles_n;           // raster: m-tiles per band (0 = all), number of n-tiles
   uint32_t mn_lbo, mn_sbo, mn_kstep;  // descriptor constants of MN-major tiles
   MmtErrorWord* ew;
+  int local_only;                 // no waits on other CTAs or peers: this launch may overlap its neighbours' ends
   // --- stream-K for the last partial wave: the final `sk_tiles` tiles are cut along K into gridDim.x equal runs of
   //     k-blocks, one per CTA; a CTA that does not reach the end of a tile leaves its fp32 partial in `sk_ws`
   //     (slot = CTA index) and raises sk_flags[CTA] to sk_epoch; the CTA that reaches the end adds the partials of
@@ -771,6 +772,7 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -855,6 +857,9 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           if (++s == kStages) { s = 0; ph ^= 1; }
         }
       }
+      // the last operand tile is on its way: CTAs of the next kernel may become resident (not earlier: from the
+      // start of a GEMM they would sit on the SMs that this grid leaves free for its whole run)
+      if (p.local_only) grid_dependents_launch();
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
@@ -1301,8 +1306,11 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tc, cons
   }
   const int tiles = ((p.M + C_::BMT - 1) / C_::BMT) * ((p.N + BN - 1) / BN);
   const int grid = (tiles < sms && p.sk_tiles == 0) ? tiles : sms;
-  gemm_bf16_tcgen05<BN, MT><<<grid, kThreads, C_::SMEM, st>>>(ta, tb, tc, p);
-  return (int)cudaGetLastError();
+  if (!p.local_only) {
+    gemm_bf16_tcgen05<BN, MT><<<grid, kThreads, C_::SMEM, st>>>(ta, tb, tc, p);
+    return (int)cudaGetLastError();
+  }
+  return (int)launch_dependent(gemm_bf16_tcgen05<BN, MT>, grid, kThreads, C_::SMEM, st, ta, tb, tc, p);
 }
 
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tc, const GemmParams& p, int sms,
@@ -1677,7 +1685,8 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
       sk_on = true;
     }
   }
-  // bf16 results leave through the epilogue warps' shared-memory slabs as full 128-byte row segments
+  // stream-K CTAs wait for one another and share a workspace: those launches keep to themselves as well
+  p.local_only = comm == nullptr && !sk_on;
   // bf16 results leave through the epilogue warps' shared-memory slabs: as bulk stores of [32 x 64] boxes
   // (tma_store == 2; a reduce-scatter producer needs rows-per-owner to be a multiple of 32 for that, so that a slab
   // has a single owner) or else as plain 16-byte stores of full row segments (tma_store == 1)
