@@ -163,8 +163,7 @@ class TextDecoder(nn.Module):
                                                               key=("text-ew", id(self)))
         if self.tp.fused is not None:
             self.tp.fused.set_checkpointed("text", ckpt)
-        one_node = (self.tp.size == 1 and torch.is_grad_enabled() and blocks.usable(x)
-                    and attn_mod.BACKEND == "sm100")
+        one_node = self.tp.size == 1 and blocks.usable(x) and attn_mod.BACKEND == "sm100"
         if one_node:
             d = self.cfg.head_dim
             spec = blocks.BlockSpec(n_q=self.n_q, n_kv=self.n_kv, head_dim=d, rope_heads=self.n_q + self.n_kv,

@@ -211,8 +211,7 @@ class VisionEncoder(nn.Module):
                                                               key=("vision-ew", id(self)))
         if self.sp.fused is not None:
             self.sp.fused.fc.set_checkpointed("vision", ckpt)
-        one_node = (torch.is_grad_enabled() and blocks.usable(x) and attn_mod.BACKEND == "sm100"
-                    and self.tp.size == 1)
+        one_node = blocks.usable(x) and attn_mod.BACKEND == "sm100" and self.tp.size == 1
         spec = blocks.BlockSpec(n_q=cfg.num_heads, n_kv=cfg.num_heads, head_dim=cfg.head_dim,
                                 rope_heads=2 * cfg.num_heads, causal=False, eps=cfg.rms_norm_eps,
                                 scale=1.0 / math.sqrt(cfg.head_dim))
@@ -227,7 +226,7 @@ class VisionEncoder(nn.Module):
                                        (B.norm1_w, B.qkv_w, B.qkv_b, B.proj_w, B.proj_b, B.norm2_w, B.gate_up_w,
                                         B.gate_up_b, B.down_w, B.down_b), recompute=ckpt, keep_elementwise=keep_ew)
                 continue
-            if one_node and is_full and getattr(self.sp.fused, "one_node", False):
+            if one_node and is_full and torch.is_grad_enabled() and getattr(self.sp.fused, "one_node", False):
                 # full attention across ranks: one node with the Ulysses exchanges inside the GEMMs
                 x = ulysses_block.ulysses_block(x, spec, plan, full_seq, self.sp.fused,
                                                 (B.norm1_w, B.qkv_w, B.qkv_b, B.proj_w, B.proj_b, B.norm2_w,

@@ -10,7 +10,7 @@ full-attention layers when one rank holds the whole image) and what the text dec
 tensor parallel.  Built from the per-op autograd functions of :mod:`.functional` under an activation
 checkpoint, such a block costs about forty graph nodes and two passes through the autograd engine per step,
 and on a B200 the HOST then needs as long to enqueue a training step as the GPU needs to run it.  This module
-issues the same kernels directly:
+issues the same kernels directly, from native code (``csrc/block.cu``: one call per block and direction):
 
 * forward keeps the block input only (activation checkpointing) or, when memory allows, also the GEMM and
   attention results;
@@ -22,13 +22,14 @@ with communication inside (Ulysses layers, tensor-parallel layers) and as the or
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 
 import torch
 
 from . import functional as F
 from . import native as nv
-from .attention import SeqInfo
+from .attention import SeqInfo, _sm_count
 
 
 @dataclass(frozen=True)
@@ -89,7 +90,6 @@ def _attn_fwd(qkv: torch.Tensor, s: BlockSpec, seq: SeqInfo):
 
 
 def _attn_bwd(qkv, out, dout, lse, s: BlockSpec, seq: SeqInfo) -> torch.Tensor:
-    from .attention import _sm_count
     T = qkv.shape[0]
     lo, hi = seq.bounds()
     dqkv = torch.empty_like(qkv)
@@ -125,21 +125,52 @@ def _linear_bwd(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, b) -> torch.
     return F.gemm(dy, w, b_mn=True)
 
 
-def _forward_chain(x, s: BlockSpec, cos, sin, seq, P, keep: bool):
-    """The block's kernels in order; with ``keep`` every intermediate the backward needs is returned."""
-    ln1_w, qkv_w, qkv_b, proj_w, proj_b, ln2_w, gu_w, gu_b, down_w, down_b = P
-    h1, rstd1 = _rmsnorm_fwd(x, ln1_w, s.eps)
-    qkv = F.gemm(h1, qkv_w, bias=qkv_b)
-    _rope_(qkv, cos, sin, s.rope_heads, s.head_dim, False)
-    a, lse = _attn_fwd(qkv, s, seq)
-    x1 = F.gemm(a, proj_w, bias=proj_b, residual=x)
-    h2, rstd2 = _rmsnorm_fwd(x1, ln2_w, s.eps)
-    gu = F.gemm(h2, gu_w, bias=gu_b)
-    m = _swiglu_fwd(gu)
-    y = F.gemm(m, down_w, bias=down_b, residual=x1)
-    if keep:
-        return y, (h1, rstd1, qkv, a, lse, x1, h2, rstd2, gu, m)
-    return y, None
+# --------------------------------------------------------------------------------------
+# Native calls: csrc/block.cu takes one array of 64-bit words (addresses, sizes, flags) in this order
+# --------------------------------------------------------------------------------------
+_N_WORDS = 10 + 6 + 10 + 8 + 10 + 1 + 2 + 4 + 3 + 1
+_Words = ctypes.c_int64 * _N_WORDS
+nv.declare("mmt_block_words", nv.c_int, [])
+nv.declare("mmt_block_fwd", nv.c_int, [nv._P, nv.c_float, nv.c_float, nv._P])
+nv.declare("mmt_block_rebuild", nv.c_int, [nv._P, nv.c_float, nv._P])
+nv.declare("mmt_block_bwd", nv.c_int, [nv._P, nv.c_float, nv._P])
+
+_ACT = ("h1", "rstd1", "qkv", "a", "lse", "x1", "h2", "rstd2", "gu", "m")
+_KEPT = {0: _ACT, 1: ("qkv", "a", "lse", "x1", "gu"), 2: ()}      # by recompute level
+
+
+def _carve(sizes, device) -> tuple[torch.Tensor, list[int]]:
+    """One byte buffer for several arrays: the buffer and their addresses, each on a 256-byte boundary."""
+    offs, total = [], 0
+    for n in sizes:
+        offs.append(total)
+        total += (n + 255) & -256
+    buf = torch.empty(total, device=device, dtype=torch.uint8)
+    base = buf.data_ptr()
+    return buf, [base + o for o in offs]
+
+
+def _act_sizes(T: int, C: int, s: BlockSpec, inter: int) -> dict[str, int]:
+    qw, aw = (s.n_q + 2 * s.n_kv) * s.head_dim, s.n_q * s.head_dim
+    return dict(h1=2 * T * C, rstd1=4 * T, qkv=2 * T * qw, a=2 * T * aw, lse=4 * s.n_q * T, x1=2 * T * C, h2=2 * T * C,
+                rstd2=4 * T, gu=4 * T * inter, m=2 * T * inter)
+
+
+def _dense(t):
+    return t if t is None or t.is_contiguous() else t.contiguous()
+
+
+def _front_words(x, y: int, P, cos, sin, seq, s: BlockSpec, act: dict, inter: int) -> list[int]:
+    lo, hi = seq.bounds()
+    T, C = x.shape
+    return [0 if p is None else p.data_ptr() for p in P] + [
+        x.data_ptr(), y, cos.data_ptr(), sin.data_ptr(), lo.data_ptr(), hi.data_ptr(), *[act[k] for k in _ACT],
+        T, C, s.n_q, s.n_kv, s.head_dim, s.rope_heads, inter, int(s.causal)]
+
+
+def _native_call(name: str, words, *args) -> None:
+    nv.call(name, ctypes.addressof(words), *args, nv.stream())
+    nv.launch_count += words[_N_WORDS - 1] - 1         # nv.call has counted one
 
 
 class _LocalBlockFn(torch.autograd.Function):
@@ -148,47 +179,87 @@ class _LocalBlockFn(torch.autograd.Function):
         # recompute: 2 = keep only the block input, 1 = also keep what is expensive to rebuild (GEMM and attention
         # results; the element-wise intermediates are recomputed from them), 0 = keep every intermediate
         x = x if x.is_contiguous() else x.contiguous()
-        y, kept = _forward_chain(x, spec, cos, sin, seq, params, keep=recompute < 2)
-        extra = ()
-        if recompute < 2:
-            h1, rstd1, qkv, a, lse, x1, h2, rstd2, gu, m = kept
-            extra = (qkv, a, lse, x1, gu) if recompute == 1 else (qkv, a, lse, x1, gu, h1, rstd1, h2, rstd2, m)
-        ctx.n_extra = len(extra)
-        ctx.save_for_backward(x, cos, sin, *extra, *[p for p in params if p is not None])
+        s = spec
+        T, C = x.shape
+        P = [_dense(p) for p in params]
+        inter, qw, aw = P[8].shape[1], (s.n_q + 2 * s.n_kv) * s.head_dim, s.n_q * s.head_dim
+        assert P[1].shape == (qw, C) and P[3].shape == (C, aw) and P[6].shape == (2 * inter, C) and P[8].shape[0] == C
+        sizes = _act_sizes(T, C, s, inter)
+        kept = _KEPT[recompute]
+        buf, addr = _carve([sizes[k] for k in kept], x.device)
+        act = dict(zip(kept, addr))
+        rest = [k for k in _ACT if k not in act]
+        tmp, addr = _carve([sizes[k] for k in rest], x.device)
+        act.update(zip(rest, addr))
+        y = torch.empty_like(x)
+        words = _Words(*_front_words(x, y.data_ptr(), P, cos, sin, seq, s, act, inter))
+        _native_call("mmt_block_fwd", words, s.eps, s.scale)
+        ctx.save_for_backward(x, cos, sin, buf, *[p for p in params if p is not None])
         ctx.has = [p is not None for p in params]
-        ctx.spec, ctx.seq = spec, seq
+        ctx.spec, ctx.seq, ctx.level = spec, seq, recompute
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        saved = ctx.saved_tensors
-        x, cos, sin = saved[0], saved[1], saved[2]
-        extra = saved[3:3 + ctx.n_extra]
-        it = iter(saved[3 + ctx.n_extra:])
-        P = tuple(next(it) if h else None for h in ctx.has)
-        s, seq = ctx.spec, ctx.seq
-        ln1_w, qkv_w, qkv_b, proj_w, proj_b, ln2_w, gu_w, gu_b, down_w, down_b = P
+        x, cos, sin, buf, *ps = ctx.saved_tensors
+        it = iter(ps)
+        params = [next(it) if h else None for h in ctx.has]
+        P = [_dense(p) for p in params]
+        s, seq, level = ctx.spec, ctx.seq, ctx.level
         dy = dy if dy.is_contiguous() else dy.contiguous()
-        if ctx.n_extra == 10:
-            qkv, a, lse, x1, gu, h1, rstd1, h2, rstd2, m = extra
-        elif ctx.n_extra:
-            qkv, a, lse, x1, gu = extra
-            h1, rstd1 = _rmsnorm_fwd(x, ln1_w, s.eps)
-            h2, rstd2 = _rmsnorm_fwd(x1, ln2_w, s.eps)
-            m = _swiglu_fwd(gu)
-        else:
-            _, (h1, rstd1, qkv, a, lse, x1, h2, rstd2, gu, m) = _forward_chain(x, s, cos, sin, seq, P, keep=True)
-        # MLP half
-        dm = _linear_bwd(dy, m, down_w, down_b)
-        dgu = _swiglu_bwd(dm, gu)
-        dh2 = _linear_bwd(dgu, h2, gu_w, gu_b)
-        dx1 = _rmsnorm_bwd(dh2, x1, ln2_w, rstd2, dy)
-        # attention half
-        da = _linear_bwd(dx1, a, proj_w, proj_b)
-        dqkv = _attn_bwd(qkv, a, da, lse, s, seq)
-        _rope_(dqkv, cos, sin, s.rope_heads, s.head_dim, True)
-        dh1 = _linear_bwd(dqkv, h1, qkv_w, qkv_b)
-        dx = _rmsnorm_bwd(dh1, x, ln1_w, rstd1, dx1)
+        T, C = x.shape
+        dev = x.device
+        inter, qw, aw = P[8].shape[1], (s.n_q + 2 * s.n_kv) * s.head_dim, s.n_q * s.head_dim
+        # the kept activations where forward laid them out, the others in a buffer of this call
+        sizes = _act_sizes(T, C, s, inter)
+        act, at = {}, buf.data_ptr()
+        for k in _KEPT[level]:
+            act[k] = at
+            at += (sizes[k] + 255) & -256
+        rest = [k for k in _ACT if k not in act]
+        tmp, addr = _carve([sizes[k] for k in rest], dev)
+        act.update(zip(rest, addr))
+        # parameter gradients: into the flat buffer where a parameter has a view of it
+        grads, flat, fresh, acc = [], [], [], 0
+        for i, p in enumerate(params):
+            mg = None if p is None else getattr(p, "main_grad", None)
+            if p is None:
+                grads.append(0)
+            elif mg is not None and mg.is_contiguous():
+                written = bool(getattr(p, "grad_written", False))
+                grads.append(mg.data_ptr())
+                acc |= int(written) << i
+                flat.append((p, mg, written))
+            else:
+                g = torch.empty(p.shape, device=dev, dtype=p.dtype)
+                fresh.append((p, mg, g))
+                grads.append(g.data_ptr())
+        parts = max(nv.lib().mmt_rmsnorm_bwd_parts(T) * C, nv.lib().mmt_colsum_parts(T) * max(2 * inter, qw, C))
+        # GQA with few KV tiles: one dK/dV CTA per q head needs an fp32 partial-sum workspace
+        split = s.n_q > s.n_kv and ((T + 127) // 128) * s.n_kv < 2 * _sm_count()
+        dx = torch.empty_like(x)
+        scratch, addr = _carve([4 * T * inter, 2 * T * max(inter, qw), 2 * T * max(C, aw), 2 * T * C, 4 * s.n_q * T,
+                                8 * s.n_q * T * s.head_dim if split else 0, 4 * parts], dev)
+        if not split:
+            addr[5] = 0
+        words = _Words(*_front_words(x, 0, P, cos, sin, seq, s, act, inter), *grads, acc, dy.data_ptr(), dx.data_ptr(),
+                       *addr)
+        if level == 2:
+            _native_call("mmt_block_fwd", words, s.eps, s.scale)
+        elif level == 1:
+            _native_call("mmt_block_rebuild", words, s.eps)
+        _native_call("mmt_block_bwd", words, s.scale)
+        if T == 0:                                # no rows, no launches: gradients that nothing wrote are zero
+            for t in [mg for _, mg, written in flat if not written] + [g for _, _, g in fresh]:
+                t.zero_()
+        for p, _, _ in flat:
+            p.grad_written = True
+        for p, mg, g in fresh:
+            if mg is None:
+                p.grad = g if p.grad is None else p.grad + g
+            else:
+                mg.copy_(mg + g if getattr(p, "grad_written", False) else g)
+                p.grad_written = True
         return (dx, None, None, None, None, None) + (None,) * len(ctx.has)
 
 
@@ -198,10 +269,10 @@ def local_block(x: torch.Tensor, spec: BlockSpec, cos: torch.Tensor, sin: torch.
     be None.  x is [T, C] bf16 on the GPU; the result has the same shape.  ``recompute``: keep only the block input
     and rebuild everything in backward (activation checkpointing); else keep the GEMM / attention results and, with
     ``keep_elementwise``, the normalised inputs and the SwiGLU output as well."""
-    level = 2 if recompute else (0 if keep_elementwise else 1)
+    level = 2 if recompute or not torch.is_grad_enabled() else (0 if keep_elementwise else 1)
     return _LocalBlockFn.apply(x, spec, cos, sin, seq, level, *params)
 
 
 def usable(x: torch.Tensor) -> bool:
-    """The fused block needs the GPU path and a gradient-carrying input (it is its own activation checkpoint)."""
+    """The fused block needs the GPU path."""
     return x.is_cuda and x.dtype == torch.bfloat16
