@@ -7,7 +7,7 @@
 // one mechanism: a query tile of 128 consecutive rows may span several (short) sequences and the
 // mask keeps every row inside its own.  GQA: q head h reads kv head h / (n_q / n_kv).
 //
-// Forward: one CTA per pair of (128-row query tile, q head) items, 10 warps (two softmax warp groups, a TMA
+// Forward: one CTA per pair of neighbouring 128-row query tiles of a q head, 10 warps (two softmax warp groups, a TMA
 // producer, an MMA issuer); see the comment at attn_fwd2_kernel.
 // head_dim 80 is not a multiple of the 64-column swizzle atom: every operand tile is fetched as two
 // 64-column boxes (columns 0-63 and 64-127 of the head; the tail of the second box belongs to the
@@ -27,42 +27,47 @@ namespace {
 using namespace attn;
 
 // ------------------------------------------------------------------------------------------------
-// Forward: two (query tile, head) items per CTA worked in ping-pong.
+// Forward: two neighbouring query tiles of one head per CTA, worked in ping-pong.
 //
-// With one item per CTA the four softmax warps are the limit: while they convert S of tile j the tensor core
-// idles.  Here a CTA owns two items, each with its own
-// softmax warp group (4 warps, one query row per thread), its own K and V buffers and its own tensor-memory
-// columns, while ONE TMA warp and ONE MMA warp serve both, so the tensor core computes S or PV of one item
-// while the other item's rows are in the exponentials.
+// With one tile per CTA the softmax warps are the limit: while they convert S of tile j the tensor core idles.  Here a
+// CTA owns two query tiles, each with its own softmax warp group (4 warps, one query row per thread) and its own
+// tensor-memory columns, while ONE TMA warp and ONE MMA warp serve both, so the tensor core computes S or PV of one
+// tile while the other tile's rows are in the exponentials.
+//   * Both tiles read the same K and V blocks (a two-stage ring): half the operand traffic of two independent tiles.
+//     A tile skips the blocks outside its own visible range (packed sequences, causal).
 //   * P never touches shared memory: the softmax threads write it as packed bf16 pairs over the first 64
 //     columns of the S tile they have just read (tcgen05.st), and PV takes it as the tensor-memory A operand.
+//   * A thread reads its 128 scores ONCE, into registers, and maximum, exponentials and sum run from there with
+//     packed fp32 pairs: per 128 x 128 tile the exponentials alone need 1024 cycles of an SM (16 per cycle), the MMAs
+//     640 (head_dim 80), so everything else has to fit beside them.  Reading
+//     the scores twice, one wait per 32 columns: 2.00 ms for one image of 16384 patches (16 heads of 80), now 1.75 ms.
 //   * O stays in tensor memory for the whole KV loop (PV accumulates).  The running maximum is lazy: O and l
 //     are rescaled only when a row's maximum grew by more than 2^8 since the value in use, which after the
 //     first tiles is rare; the rescale is a tensor-memory read-modify-write by the row's own thread, safe
 //     because S of tile j is only published after PV of tile j-1 has completed.
 //   * KV tiles that are entirely visible to every row of a warp skip the per-element mask.
-// Tensor memory: S/P of item w at columns [128w, 128w+128), O of item w at [256+128w, 256+128w+DIM).
-// Shared memory: Q, K, V of each item, 32 KB each (two 64-column boxes).
+// Tensor memory: S/P of tile w at columns [128w, 128w+128), O of tile w at [256+128w, 256+128w+DIM).
+// Shared memory: Q of each tile and two stages of K and V, 32 KB each (two 64-column boxes).
 // ------------------------------------------------------------------------------------------------
 constexpr int kFwd2Threads = 320;
 
 template <int DIM>
 __global__ void __launch_bounds__(kFwd2Threads, 1)
-attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, const int n_items) {
+attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, const int n_pairs) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;                         // [item][2 boxes]
-  uint8_t* sK = sQ + 4 * CHUNK;
+  uint8_t* sQ = smem;                         // [tile][2 boxes]
+  uint8_t* sK = sQ + 4 * CHUNK;               // [stage][2 boxes]
   uint8_t* sV = sK + 4 * CHUNK;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 4 * CHUNK);
-  uint64_t* q_full = bars;          // [2]
-  uint64_t* k_full = bars + 2;      // [2]
-  uint64_t* k_empty = bars + 4;     // [2]
-  uint64_t* v_full = bars + 6;      // [2]
-  uint64_t* v_empty = bars + 8;     // [2]
-  uint64_t* s_full = bars + 10;     // [2]
-  uint64_t* p_full = bars + 12;     // [2]
-  uint64_t* pv_done = bars + 14;    // [2]
+  uint64_t* q_full = bars;          // [2] per tile
+  uint64_t* k_full = bars + 2;      // [2] per stage
+  uint64_t* k_empty = bars + 4;     // [2] per stage
+  uint64_t* v_full = bars + 6;      // [2] per stage
+  uint64_t* v_empty = bars + 8;     // [2] per stage
+  uint64_t* s_full = bars + 10;     // [2] per tile
+  uint64_t* p_full = bars + 12;     // [2] per tile
+  uint64_t* pv_done = bars + 14;    // [2] per tile
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -91,57 +96,49 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   grid_dependency_sync();
-  // the two items of this CTA: heads fastest, so both usually share the query rows (and, with GQA, K and V)
-  int q0[2], head[2], kv_lo[2], n_tiles[2], xq[2], xk[2], xv[2];
+  // non-causal: the CTAs that run together share a head, so its K and V stay in L2 however long the sequence;
+  // causal: the last query tiles see the most KV blocks and are started first, over all heads (longest work first)
+  const int head = p.causal ? (int)blockIdx.x % p.n_q : (int)blockIdx.x / n_pairs;
+  const int pair = p.causal ? n_pairs - 1 - (int)blockIdx.x / p.n_q : (int)blockIdx.x % n_pairs;
+  const int kv_head = head / (p.n_q / p.n_kv);
+  const int xq = head * DIM, xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
+  // blocks j in [first[w], last[w]) of 128 KV rows, counted from the first row that tile 0 sees, are visible to tile w
+  int q0[2], first[2], last[2];
+  int kv_base = 0;
 #pragma unroll
   for (int w = 0; w < 2; ++w) {
-    // causal: the last query tiles see the most KV tiles, so they are started first (longest work first)
-    const int cta = p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
-    const int item = cta * 2 + w;
-    n_tiles[w] = 0;
-    q0[w] = head[w] = kv_lo[w] = xq[w] = xk[w] = xv[w] = 0;
-    if (item < n_items) {
-      head[w] = item % p.n_q;
-      q0[w] = (item / p.n_q) * BQ;
-      const int kv_head = head[w] / (p.n_q / p.n_kv);
+    q0[w] = (pair * 2 + w) * BQ;
+    first[w] = last[w] = 0;
+    if (q0[w] < p.T) {
       const int q_last = min(q0[w] + BQ, p.T) - 1;
-      kv_lo[w] = p.seq_lo[q0[w]];
-      const int kv_hi = p.causal ? min(p.seq_hi[q_last], q_last + 1) : p.seq_hi[q_last];
-      n_tiles[w] = (kv_hi - kv_lo[w] + BKV - 1) / BKV;
-      xq[w] = head[w] * DIM;
-      xk[w] = (p.n_q + kv_head) * DIM;
-      xv[w] = (p.n_q + p.n_kv + kv_head) * DIM;
+      const int lo = p.seq_lo[q0[w]];
+      const int hi = p.causal ? min(p.seq_hi[q_last], q_last + 1) : p.seq_hi[q_last];
+      if (w == 0) kv_base = lo;
+      first[w] = (lo - kv_base) / BKV;
+      last[w] = (hi - kv_base + BKV - 1) / BKV;
     }
   }
-  const int max_tiles = max(n_tiles[0], n_tiles[1]);
+  const int n_blocks = max(last[0], last[1]);
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
+      auto load = [&](uint8_t* dst, uint64_t* bar, int x, int y) {
+        mbar_expect_tx(bar, 2 * CHUNK);
+        tma_load_2d(dst, &tm, bar, x, y);
+        tma_load_2d(dst + CHUNK, &tm, bar, x + X2, y);
+      };
       bool ok = true;
-      for (int w = 0; w < 2; ++w) {
-        if (n_tiles[w] == 0) continue;
-        mbar_expect_tx(&q_full[w], 2 * CHUNK);
-        tma_load_2d(sQ + w * 2 * CHUNK, &tm, &q_full[w], xq[w], q0[w]);
-        tma_load_2d(sQ + w * 2 * CHUNK + CHUNK, &tm, &q_full[w], xq[w] + X2, q0[w]);
-      }
-      for (int j = 0; j < max_tiles && ok; ++j) {
-        for (int w = 0; w < 2 && ok; ++w) {
-          if (j >= n_tiles[w]) continue;
-          if (j > 0 && !mbar_wait(&k_empty[w], (j - 1) & 1, p.ew, 410)) { ok = false; break; }
-          const int r0 = kv_lo[w] + j * BKV;
-          mbar_expect_tx(&k_full[w], 2 * CHUNK);
-          tma_load_2d(sK + w * 2 * CHUNK, &tm, &k_full[w], xk[w], r0);
-          tma_load_2d(sK + w * 2 * CHUNK + CHUNK, &tm, &k_full[w], xk[w] + X2, r0);
-        }
-        for (int w = 0; w < 2 && ok; ++w) {
-          if (j >= n_tiles[w]) continue;
-          if (j > 0 && !mbar_wait(&v_empty[w], (j - 1) & 1, p.ew, 411)) { ok = false; break; }
-          const int r0 = kv_lo[w] + j * BKV;
-          mbar_expect_tx(&v_full[w], 2 * CHUNK);
-          tma_load_2d(sV + w * 2 * CHUNK, &tm, &v_full[w], xv[w], r0);
-          tma_load_2d(sV + w * 2 * CHUNK + CHUNK, &tm, &v_full[w], xv[w] + X2, r0);
-        }
+      if (last[0] > first[0]) load(sQ, &q_full[0], xq, q0[0]);
+      for (int j = 0; j < n_blocks && ok; ++j) {
+        const int st = j & 1;
+        const uint32_t free_parity = (uint32_t)(((j >> 1) & 1) ^ 1);
+        const int r0 = kv_base + j * BKV;
+        if (!mbar_wait(&k_empty[st], free_parity, p.ew, 410)) { ok = false; break; }
+        load(sK + st * 2 * CHUNK, &k_full[st], xk, r0);
+        if (j == 0 && last[1] > first[1]) load(sQ + 2 * CHUNK, &q_full[1], xq, q0[1]);
+        if (!mbar_wait(&v_empty[st], free_parity, p.ew, 411)) { ok = false; break; }
+        load(sV + st * 2 * CHUNK, &v_full[st], xv, r0);
       }
     }
   } else if (warp == 9) {
@@ -149,55 +146,67 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
     if (lane == 0) {
       const uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
       const uint32_t idesc_pv = make_idesc_bf16(BQ, DIM, 0, 1);
-      const uint32_t hi_k = smem_desc_hi(1024), hi_v = smem_desc_hi(1024);
-      uint32_t q_lo[2], k_lo[2], v_lo[2];
-      for (int w = 0; w < 2; ++w) {
-        q_lo[w] = smem_desc_lo(smem_u32(sQ + w * 2 * CHUNK), 16);
-        k_lo[w] = smem_desc_lo(smem_u32(sK + w * 2 * CHUNK), 16);
-        v_lo[w] = smem_desc_lo(smem_u32(sV + w * 2 * CHUNK), CHUNK);
-      }
-      auto issue_s = [&](int w) {
+      const uint32_t hi = smem_desc_hi(1024);
+      const uint32_t q_lo = smem_desc_lo(smem_u32(sQ), 16);
+      const uint32_t k_lo = smem_desc_lo(smem_u32(sK), 16);
+      const uint32_t v_lo = smem_desc_lo(smem_u32(sV), CHUNK);
+      constexpr uint32_t kPair = (2 * CHUNK) >> 4;      // one tile's or stage's two boxes
+      auto issue_s = [&](int w, int j) {
         const uint32_t d = tmem_base + (uint32_t)(w * 128);
+        const uint32_t a = q_lo + (uint32_t)w * kPair, b = k_lo + (uint32_t)(j & 1) * kPair;
 #pragma unroll
         for (int k = 0; k < DIM / 16; ++k) {
           const uint32_t off = (uint32_t)(((k >> 2) * CHUNK + (k & 3) * 32) >> 4);
-          tc_mma_ss(d, smem_desc_join(hi_k, q_lo[w] + off), smem_desc_join(hi_k, k_lo[w] + off), idesc_s, k != 0);
+          tc_mma_ss(d, smem_desc_join(hi, a + off), smem_desc_join(hi, b + off), idesc_s, k != 0);
         }
         tc_commit(&s_full[w]);
-        tc_commit(&k_empty[w]);
       };
+      auto sees = [&](int w, int j) { return j >= first[w] && j < last[w]; };
+      int seen[2] = {0, 0};                             // blocks of tile w whose P has been consumed
       bool ok = true;
+      if (n_blocks > 0) ok = mbar_wait(&k_full[0], 0, p.ew, 511);
       for (int w = 0; w < 2 && ok; ++w) {
-        if (n_tiles[w] == 0) continue;
-        ok = mbar_wait(&q_full[w], 0, p.ew, 510) && mbar_wait(&k_full[w], 0, p.ew, 511);
-        if (ok) issue_s(w);
+        if (!sees(w, 0)) continue;
+        ok = mbar_wait(&q_full[w], 0, p.ew, 510);
+        if (ok) issue_s(w, 0);
       }
-      for (int j = 0; j < max_tiles && ok; ++j) {
+      if (ok && n_blocks > 0) tc_commit(&k_empty[0]);
+      for (int j = 0; j < n_blocks && ok; ++j) {
+        const int nx = j + 1;
+        bool have_k = false, have_v = false;
         for (int w = 0; w < 2 && ok; ++w) {
-          if (j >= n_tiles[w]) continue;
-          if (!mbar_wait(&p_full[w], j & 1, p.ew, 512) || !mbar_wait(&v_full[w], j & 1, p.ew, 513)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t d = tmem_base + 256u + (uint32_t)(w * 128);
-          const uint32_t a = tmem_base + (uint32_t)(w * 128);
+          if (sees(w, j)) {
+            if (!have_v && !mbar_wait(&v_full[j & 1], (j >> 1) & 1, p.ew, 513)) { ok = false; break; }
+            have_v = true;
+            if (!mbar_wait(&p_full[w], seen[w] & 1, p.ew, 512)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t d = tmem_base + 256u + (uint32_t)(w * 128);
+            const uint32_t a = tmem_base + (uint32_t)(w * 128);
+            const uint32_t b = v_lo + (uint32_t)(j & 1) * kPair;
 #pragma unroll
-          for (int k = 0; k < BKV / 16; ++k) {
-            tc_mma_ts(d, a + (uint32_t)(k * 8), smem_desc_join(hi_v, v_lo[w] + (uint32_t)(k * (2048 >> 4))), idesc_pv,
-                      (j | k) != 0);
+            for (int k = 0; k < BKV / 16; ++k)
+              tc_mma_ts(d, a + (uint32_t)(k * 8), smem_desc_join(hi, b + (uint32_t)(k * (2048 >> 4))), idesc_pv,
+                        (seen[w] | k) != 0);
+            ++seen[w];
+            if (j == last[w] - 1) tc_commit(&pv_done[w]);
           }
-          tc_commit(&v_empty[w]);
-          if (j == n_tiles[w] - 1) tc_commit(&pv_done[w]);
-          if (j + 1 < n_tiles[w]) {
-            if (!mbar_wait(&k_full[w], (j + 1) & 1, p.ew, 514)) { ok = false; break; }
-            issue_s(w);
+          if (w == 1) tc_commit(&v_empty[j & 1]);
+          if (sees(w, nx)) {
+            if (!have_k && !mbar_wait(&k_full[nx & 1], (nx >> 1) & 1, p.ew, 514)) { ok = false; break; }
+            have_k = true;
+            if (nx == first[w] && !mbar_wait(&q_full[w], 0, p.ew, 515)) { ok = false; break; }
+            issue_s(w, nx);
           }
         }
+        if (ok && nx < n_blocks) tc_commit(&k_empty[nx & 1]);
       }
     }
   } else {
-    // ------------------------------ softmax + epilogue, one warp group per item ------------------------------
-    const int w = warp >> 2;             // item
+    // ------------------------------ softmax + epilogue, one warp group per tile ------------------------------
+    const int w = warp >> 2;             // tile
     const int q = warp & 3;              // tensor-memory lane quadrant of this warp
-    if (n_tiles[w] > 0) {
+    const int j0 = first[w], j1 = last[w];
+    if (j1 > j0) {
       const int row = q * 32 + lane;
       const int qrow = q0[w] + row;
       const bool row_ok = qrow < p.T;
@@ -205,85 +214,81 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
       int hi = row_ok ? p.seq_hi[qrow] : 0;
       if (p.causal) hi = min(hi, qrow + 1);
       const float sl2 = p.scale * LOG2E;
+      const float2 sl2_2 = make_float2(sl2, sl2);
       const uint32_t lane_addr = ((uint32_t)(q * 32) << 16);
       const uint32_t s_addr = tmem_base + lane_addr + (uint32_t)(w * 128);
       const uint32_t o_addr = tmem_base + lane_addr + 256u + (uint32_t)(w * 128);
       float m_ref = -INFINITY, l = 0.f;
       bool ok = true;
-      for (int j = 0; j < n_tiles[w]; ++j) {
-        const int kv0 = kv_lo[w] + j * BKV;
-        ok = __all_sync(0xffffffffu, mbar_wait(&s_full[w], j & 1, p.ew, 610));
+      for (int j = j0; j < j1; ++j) {
+        const int kv0 = kv_base + j * BKV;
+        ok = __all_sync(0xffffffffu, mbar_wait(&s_full[w], (j - j0) & 1, p.ew, 610));
         if (!ok) break;
         tc_fence_after();
+        uint32_t r[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(s_addr + c * 32, r[c]);
         const bool full = __all_sync(0xffffffffu, kv0 >= lo && kv0 + BKV <= hi);
-        // pass 1: row maximum over the visible columns
-        float mx = -INFINITY;
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(s_addr + c * 32, r);
-          tmem_wait_ld();
-          if (full) {
+        tmem_wait_ld();
+        // row maximum over the visible columns
+        uint32_t vis[4];
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        if (full) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
-          } else {
+          for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int kv = kv0 + c * 32 + i;
-              if (kv >= lo && kv < hi) mx = fmaxf(mx, __uint_as_float(r[i]));
-            }
+            for (int i = 0; i < 32; i += 2)
+              mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])));
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            vis[c] = visible_bits(lo - (kv0 + c * 32), hi - (kv0 + c * 32));
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              mx4[c] = fmaxf(mx4[c], (vis[c] >> i) & 1u ? __uint_as_float(r[c][i]) : -INFINITY);
           }
         }
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         // lazy running maximum: adopt a new reference only when it moved by more than 2^8
         const float m_new = fmaxf(m_ref, mx);
         const bool need = (m_new - m_ref) * sl2 > 8.f;        // false when both are -inf (NaN compares false)
-        if (j == 0) {
+        if (j == j0) {
           if (need) m_ref = m_new;                             // O does not exist yet: nothing to rescale
         } else if (__any_sync(0xffffffffu, need)) {
           const float alpha = need ? exp2f((m_ref - m_new) * sl2) : 1.f;   // exp2(-inf) = 0 for a row without history
           l *= alpha;
           if (need) m_ref = m_new;
-#pragma unroll
+#pragma unroll 1
           for (int c = 0; c < DIM / 16; ++c) {
-            uint32_t r[16];
-            tmem_ld_32x32b_x16(o_addr + c * 16, r);
+            uint32_t o[16];
+            tmem_ld_32x32b_x16(o_addr + c * 16, o);
             tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-            tmem_st_32x32b_x16(o_addr + c * 16, r);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x32b_x16(o_addr + c * 16, o);
           }
-          tmem_wait_st();
         }
         const float bias = (m_ref == -INFINITY) ? 0.f : -m_ref * sl2;
-        // pass 2: P = exp2(S * sl2 + bias) as bf16 pairs, written over the columns of S already consumed
-        float sum = 0.f;
-#pragma unroll 1
+        const float2 bias2 = make_float2(bias, bias);
+        // P = exp2(S * sl2 + bias) as bf16 pairs, written over the columns of S
+        float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(s_addr + c * 32, r);
-          tmem_wait_ld();
           uint32_t pk[16];
-          if (full) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              const float p0 = exp2f(fmaf(__uint_as_float(r[i]), sl2, bias));
-              const float p1 = exp2f(fmaf(__uint_as_float(r[i + 1]), sl2, bias));
-              sum += p0 + p1;
-              pk[i >> 1] = pack_bf16x2(p0, p1);
+          for (int i = 0; i < 32; i += 2) {
+            const float2 t = fma2(make_float2(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])), sl2_2, bias2);
+            float2 e = make_float2(exp2f(t.x), exp2f(t.y));
+            if (!full) {
+              if (!((vis[c] >> i) & 1u)) e.x = 0.f;
+              if (!((vis[c] >> (i + 1)) & 1u)) e.y = 0.f;
             }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              const int kv = kv0 + c * 32 + i;
-              const float p0 = (kv >= lo && kv < hi) ? exp2f(fmaf(__uint_as_float(r[i]), sl2, bias)) : 0.f;
-              const float p1 = (kv + 1 >= lo && kv + 1 < hi) ? exp2f(fmaf(__uint_as_float(r[i + 1]), sl2, bias)) : 0.f;
-              sum += p0 + p1;
-              pk[i >> 1] = pack_bf16x2(p0, p1);
-            }
+            sum = add2(sum, e);
+            pk[i >> 1] = pack_bf16x2(e.x, e.y);
           }
           tmem_st_32x32b_x16(s_addr + c * 16, pk);
         }
-        l += sum;
+        l += sum.x + sum.y;
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -293,27 +298,22 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
       if (ok) {
         tc_fence_after();
         const float inv = l > 0.f ? 1.f / l : 0.f;
-        __nv_bfloat16* dst = p.out + (long)qrow * (p.n_q * DIM) + head[w] * DIM;
+        __nv_bfloat16* dst = p.out + (long)qrow * (p.n_q * DIM) + head * DIM;
 #pragma unroll
         for (int c = 0; c < DIM / 16; ++c) {
-          uint32_t r[16];
-          tmem_ld_32x32b_x16(o_addr + c * 16, r);
+          uint32_t o[16];
+          tmem_ld_32x32b_x16(o_addr + c * 16, o);
           tmem_wait_ld();
           if (row_ok) {
-            uint4 v0, v1;
-            v0.x = pack_bf16x2(__uint_as_float(r[0]) * inv, __uint_as_float(r[1]) * inv);
-            v0.y = pack_bf16x2(__uint_as_float(r[2]) * inv, __uint_as_float(r[3]) * inv);
-            v0.z = pack_bf16x2(__uint_as_float(r[4]) * inv, __uint_as_float(r[5]) * inv);
-            v0.w = pack_bf16x2(__uint_as_float(r[6]) * inv, __uint_as_float(r[7]) * inv);
-            v1.x = pack_bf16x2(__uint_as_float(r[8]) * inv, __uint_as_float(r[9]) * inv);
-            v1.y = pack_bf16x2(__uint_as_float(r[10]) * inv, __uint_as_float(r[11]) * inv);
-            v1.z = pack_bf16x2(__uint_as_float(r[12]) * inv, __uint_as_float(r[13]) * inv);
-            v1.w = pack_bf16x2(__uint_as_float(r[14]) * inv, __uint_as_float(r[15]) * inv);
-            *reinterpret_cast<uint4*>(dst + c * 16) = v0;
-            *reinterpret_cast<uint4*>(dst + c * 16 + 8) = v1;
+            uint32_t v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              v[i] = pack_bf16x2(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
+            *reinterpret_cast<uint4*>(dst + c * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<uint4*>(dst + c * 16 + 8) = make_uint4(v[4], v[5], v[6], v[7]);
           }
         }
-        if (row_ok) p.lse[(long)head[w] * p.T + qrow] = l > 0.f ? m_ref * p.scale + logf(l) : INFINITY;
+        if (row_ok) p.lse[(long)head * p.T + qrow] = l > 0.f ? m_ref * p.scale + logf(l) : INFINITY;
       }
     }
   }
@@ -334,9 +334,8 @@ int launch_fwd2(const CUtensorMap& tm, const AttnParams& p, cudaStream_t st) {
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  const int n_items = ((p.T + BQ - 1) / BQ) * p.n_q;
-  launch_dependent(attn_fwd2_kernel<DIM>, (n_items + 1) / 2, kFwd2Threads, kFwdSmem, st,
-                     tm, p, n_items);
+  const int n_pairs = ((p.T + BQ - 1) / BQ + 1) / 2;
+  launch_dependent(attn_fwd2_kernel<DIM>, n_pairs * p.n_q, kFwd2Threads, kFwdSmem, st, tm, p, n_pairs);
   return (int)cudaGetLastError();
 }
 

@@ -51,4 +51,59 @@ MMT_DEVICE uint64_t desc_kmajor(uint32_t base, int k) { return make_smem_desc(km
 // MN-major operand tile: rows are the K dimension (16 rows per step), columns the M/N dimension
 MMT_DEVICE uint64_t desc_mnmajor(uint32_t base, int k) { return make_smem_desc(base + k * 2048, CHUNK, 1024); }
 
+// The two warps that share a lane quadrant (barriers 1 .. 4): both have read their columns of a score stage before
+// either writes P / dS over them.  Nothing else ties the softmax warps together inside a block, so the four pairs drift
+// apart and one pair's exponentials run beside another pair's tensor-memory traffic.
+MMT_DEVICE void pair_bar_sync(int quadrant) { asm volatile("bar.sync %0, 64;" ::"r"(quadrant + 1) : "memory"); }
+
+// Bits i of [lo, hi) within a chunk of 32 columns (lo and hi relative to the chunk's first column).
+MMT_DEVICE uint32_t visible_bits(int lo, int hi) {
+  const uint32_t below_hi = hi >= 32 ? 0xffffffffu : (hi <= 0 ? 0u : (1u << hi) - 1u);
+  const uint32_t below_lo = lo >= 32 ? 0xffffffffu : (lo <= 0 ? 0u : (1u << lo) - 1u);
+  return below_hi & ~below_lo;
+}
+
+// Two fp32 operations in one instruction (same rounding as the scalar ones).
+MMT_DEVICE float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t"
+      ".reg .b64 a, b, c, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 b, {%4, %5};\n\t"
+      "mov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t"
+      "}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+MMT_DEVICE float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t"
+      ".reg .b64 a, b, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 b, {%4, %5};\n\t"
+      "add.rn.f32x2 d, a, b;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t"
+      "}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
+MMT_DEVICE float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t"
+      ".reg .b64 a, b, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 d, a, b;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t"
+      "}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
 }  // namespace attn
