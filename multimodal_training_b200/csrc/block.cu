@@ -21,6 +21,10 @@ int mmt_colsum(const void*, void*, float*, long, int, long, int, void*);
 int mmt_gemm_bf16(const void*, const void*, void*, const void*, const void*, int, int, int, int, int, int, int, int, int,
                   int, int, int, float, int, void*);
 int mmt_attn_fwd(const void*, void*, float*, const int*, const int*, long, int, int, int, long, int, float, void*);
+int mmt_attn_local_fwd(const void*, void*, float*, const int*, const int*, const int*, int, long, int, int, int, long,
+                       int, float, void*);
+int mmt_attn_local_bwd(const void*, const void*, const void*, const float*, void*, const int*, const int*, const int*, int,
+                       long, int, int, int, long, int, float, void*);
 int mmt_attn_bwd(const void*, const void*, const void*, const float*, float*, void*, const int*, const int*, long, int,
                  int, int, long, int, float, float*, void*);
 }
@@ -36,6 +40,8 @@ struct BlockArgs {
   uint64_t cos, sin, lo, hi;
   uint64_t h1, rstd1, qkv, a, lse, x1, h2, rstd2, gu, m;   // activations [T, ...]; backward reads them
   int64_t T, C, n_q, n_kv, dim, rope_heads, inter, causal;
+  uint64_t packs;                // packs of short sequences, or 0
+  int64_t n_packs;
   // backward only
   uint64_t g[N_WEIGHTS];
   int64_t accumulate;            // bit i: add to g[i]
@@ -114,7 +120,10 @@ int mmt_block_fwd(int64_t* words, float eps, float scale, void* stream) {
   s.norm(b.x, LN1, b.h1, b.rstd1, eps);
   s.linear(b.h1, b.w[QKV_W], b.w[QKV_B], 0, b.qkv, qw, b.C);
   s.rope(b.qkv, 0);
-  if (!s.rc)
+  if (!s.rc && b.packs)
+    s.done(mmt_attn_local_fwd(s.p(b.qkv), s.p(b.a), s.f(b.lse), s.i(b.lo), s.i(b.hi), s.i(b.packs), (int)b.n_packs, b.T,
+                              (int)b.n_q, (int)b.n_kv, (int)b.dim, qw, (int)b.causal, scale, stream), 1);
+  else if (!s.rc)
     s.done(mmt_attn_fwd(s.p(b.qkv), s.p(b.a), s.f(b.lse), s.i(b.lo), s.i(b.hi), b.T, (int)b.n_q, (int)b.n_kv, (int)b.dim,
                         qw, (int)b.causal, scale, stream), 1);
   s.linear(b.a, b.w[PROJ_W], b.w[PROJ_B], b.x, b.x1, b.C, aw);
@@ -153,7 +162,11 @@ int mmt_block_bwd(int64_t* words, float scale, void* stream) {
   s.norm_bwd(b.mid, b.x1, LN2, b.rstd2, b.dy, b.dx1);
   // attention half
   s.linear_bwd(b.dx1, b.a, PROJ_W, b.mid, b.C, aw);
-  if (!s.rc)
+  if (!s.rc && b.packs && b.n_q == b.n_kv)
+    s.done(mmt_attn_local_bwd(s.p(b.qkv), s.p(b.a), s.p(b.mid), s.f(b.lse), s.p(b.big), s.i(b.lo), s.i(b.hi),
+                              s.i(b.packs), (int)b.n_packs, b.T, (int)b.n_q, (int)b.n_kv, (int)b.dim, qw, (int)b.causal,
+                              scale, stream), 1);
+  else if (!s.rc)
     s.done(mmt_attn_bwd(s.p(b.qkv), s.p(b.a), s.p(b.mid), s.f(b.lse), s.f(b.delta), s.p(b.big), s.i(b.lo), s.i(b.hi), b.T,
                         (int)b.n_q, (int)b.n_kv, (int)b.dim, qw, (int)b.causal, scale, s.f(b.ws), stream),
            b.ws ? 4 : 3);

@@ -17,6 +17,7 @@ import torch
 from . import native as nv
 
 BACKEND = "sm100"
+LOCAL_ROWS = 128      # rows of one tile: batches of sequences up to this length take csrc/attention_local.cu
 
 
 def set_backend(name: str) -> None:
@@ -35,6 +36,7 @@ class SeqInfo:
     _cu: torch.Tensor | None = None
     _lo: torch.Tensor | None = None
     _hi: torch.Tensor | None = None
+    _packs: torch.Tensor | None = None
 
     @classmethod
     def from_list(cls, cu: list[int], device) -> "SeqInfo":
@@ -64,6 +66,28 @@ class SeqInfo:
             self._lo = lo.to(self.device, non_blocking=True)
             self._hi = hi.to(self.device, non_blocking=True)
         return self._lo, self._hi
+
+
+    def packs(self) -> torch.Tensor | None:
+        """(first row, rows) of consecutive whole sequences taken together up to LOCAL_ROWS rows (int32, device), or
+        None when a sequence is longer than that: what the kernels for short sequences work on."""
+        if self._packs is None and 0 < self.max_len <= LOCAL_ROWS:
+            self._packs = torch.tensor(pack_sequences(self.host, LOCAL_ROWS), dtype=torch.int32).to(
+                self.device, non_blocking=True)
+        return self._packs
+
+
+def pack_sequences(cu: list[int], limit: int) -> list[tuple[int, int]]:
+    """Cuts the rows of ``cu`` at sequence boundaries into pieces of at most ``limit`` rows (no sequence is longer)."""
+    out = []
+    first = cu[0]
+    for a, b in zip(cu[:-1], cu[1:]):
+        if b - first > limit:
+            out.append((first, a - first))
+            first = a
+    if cu[-1] > first:
+        out.append((first, cu[-1] - first))
+    return out
 
 
 class _LibAttentionFn(torch.autograd.Function):
@@ -99,15 +123,51 @@ class _LibAttentionFn(torch.autograd.Function):
         return dqkv, None, None, None, None, None, None
 
 
+def attn_fwd(qkv: torch.Tensor, n_q: int, n_kv: int, dim: int, info: SeqInfo, causal: bool, scale: float):
+    """(out [T, n_q * dim], log-sum-exp [n_q, T])"""
+    T = qkv.shape[0]
+    lo, hi = info.bounds()
+    out = torch.empty(T, n_q * dim, device=qkv.device, dtype=qkv.dtype)
+    lse = torch.empty(n_q, T, device=qkv.device, dtype=torch.float32)
+    packs = info.packs()
+    if packs is not None:
+        nv.call("mmt_attn_local_fwd", qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), lo.data_ptr(), hi.data_ptr(),
+                packs.data_ptr(), packs.shape[0], T, n_q, n_kv, dim, qkv.stride(0), int(causal), scale, nv.stream())
+    else:
+        nv.call("mmt_attn_fwd", qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), lo.data_ptr(), hi.data_ptr(), T,
+                n_q, n_kv, dim, qkv.stride(0), int(causal), scale, nv.stream())
+    return out, lse
+
+
+def split_heads(T: int, n_q: int, n_kv: int) -> bool:
+    """GQA with few KV tiles: one dK/dV CTA per q head, which needs an fp32 partial-sum workspace."""
+    return n_q > n_kv and ((T + 127) // 128) * n_kv < 2 * _sm_count()
+
+
+def attn_bwd(qkv, out, dout, lse, n_q: int, n_kv: int, dim: int, info: SeqInfo, causal: bool, scale: float):
+    T = qkv.shape[0]
+    lo, hi = info.bounds()
+    dqkv = torch.empty_like(qkv)
+    packs = info.packs() if n_q == n_kv else None
+    if packs is not None:
+        nv.call("mmt_attn_local_bwd", qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), dqkv.data_ptr(),
+                lo.data_ptr(), hi.data_ptr(), packs.data_ptr(), packs.shape[0], T, n_q, n_kv, dim, qkv.stride(0),
+                int(causal), scale, nv.stream())
+        return dqkv
+    delta = torch.empty(n_q, T, device=qkv.device, dtype=torch.float32)
+    ws = None
+    if split_heads(T, n_q, n_kv):
+        ws = torch.empty(2 * n_q * T * dim, device=qkv.device, dtype=torch.float32)
+    nv.call("mmt_attn_bwd", qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), delta.data_ptr(),
+            dqkv.data_ptr(), lo.data_ptr(), hi.data_ptr(), T, n_q, n_kv, dim, qkv.stride(0), int(causal), scale,
+            nv.ptr(ws), nv.stream())
+    return dqkv
+
+
 class _Sm100AttentionFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, n_q, n_kv, dim, info, causal, scale):
-        T = qkv.shape[0]
-        lo, hi = info.bounds()
-        out = torch.empty(T, n_q * dim, device=qkv.device, dtype=qkv.dtype)
-        lse = torch.empty(n_q, T, device=qkv.device, dtype=torch.float32)
-        nv.call("mmt_attn_fwd", qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), lo.data_ptr(), hi.data_ptr(), T,
-                n_q, n_kv, dim, qkv.stride(0), int(causal), scale, nv.stream())
+        out, lse = attn_fwd(qkv, n_q, n_kv, dim, info, causal, scale)
         ctx.save_for_backward(qkv, out, lse)
         ctx.meta = (n_q, n_kv, dim, info, causal, scale)
         return out
@@ -115,21 +175,8 @@ class _Sm100AttentionFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         qkv, out, lse = ctx.saved_tensors
-        n_q, n_kv, dim, info, causal, scale = ctx.meta
-        T = qkv.shape[0]
-        lo, hi = info.bounds()
         dout = dout if dout.is_contiguous() else dout.contiguous()
-        dqkv = torch.empty_like(qkv)
-        delta = torch.empty(n_q, T, device=qkv.device, dtype=torch.float32)
-        # GQA with few KV tiles: one dK/dV CTA per q head needs an fp32 partial-sum workspace
-        tiles = (T + 127) // 128
-        ws = None
-        if n_q > n_kv and tiles * n_kv < 2 * _sm_count():
-            ws = torch.empty(2 * n_q * T * dim, device=qkv.device, dtype=torch.float32)
-        nv.call("mmt_attn_bwd", qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), delta.data_ptr(),
-                dqkv.data_ptr(), lo.data_ptr(), hi.data_ptr(), T, n_q, n_kv, dim, qkv.stride(0), int(causal), scale,
-                nv.ptr(ws), nv.stream())
-        return dqkv, None, None, None, None, None, None
+        return (attn_bwd(qkv, out, dout, lse, *ctx.meta),) + (None,) * 6
 
 
 def flash_attention(qkv: torch.Tensor, n_q: int, n_kv: int, dim: int, info: SeqInfo, causal: bool,
@@ -144,6 +191,10 @@ nv.declare("mmt_attn_fwd", nv.c_int, [nv._P, nv._P, nv._P, nv._P, nv._P, nv.c_lo
                                       nv.c_long, nv.c_int, nv.c_float, nv._P])
 nv.declare("mmt_attn_bwd", nv.c_int, [nv._P, nv._P, nv._P, nv._P, nv._P, nv._P, nv._P, nv._P, nv.c_long, nv.c_int,
                                       nv.c_int, nv.c_int, nv.c_long, nv.c_int, nv.c_float, nv._P, nv._P])
+nv.declare("mmt_attn_local_fwd", nv.c_int, [nv._P, nv._P, nv._P, nv._P, nv._P, nv._P, nv.c_int, nv.c_long, nv.c_int,
+                                            nv.c_int, nv.c_int, nv.c_long, nv.c_int, nv.c_float, nv._P])
+nv.declare("mmt_attn_local_bwd", nv.c_int, [nv._P, nv._P, nv._P, nv._P, nv._P, nv._P, nv._P, nv._P, nv.c_int, nv.c_long,
+                                            nv.c_int, nv.c_int, nv.c_int, nv.c_long, nv.c_int, nv.c_float, nv._P])
 
 
 def _sm_count() -> int:

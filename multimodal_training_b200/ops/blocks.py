@@ -29,7 +29,7 @@ import torch
 
 from . import functional as F
 from . import native as nv
-from .attention import SeqInfo, _sm_count
+from .attention import SeqInfo, attn_bwd, attn_fwd, split_heads
 
 
 @dataclass(frozen=True)
@@ -80,27 +80,11 @@ def _rope_(t: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, heads: int, di
 
 
 def _attn_fwd(qkv: torch.Tensor, s: BlockSpec, seq: SeqInfo):
-    T = qkv.shape[0]
-    lo, hi = seq.bounds()
-    out = torch.empty(T, s.n_q * s.head_dim, device=qkv.device, dtype=qkv.dtype)
-    lse = torch.empty(s.n_q, T, device=qkv.device, dtype=torch.float32)
-    nv.call("mmt_attn_fwd", qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), lo.data_ptr(), hi.data_ptr(), T, s.n_q,
-            s.n_kv, s.head_dim, qkv.stride(0), int(s.causal), s.scale, nv.stream())
-    return out, lse
+    return attn_fwd(qkv, s.n_q, s.n_kv, s.head_dim, seq, s.causal, s.scale)
 
 
 def _attn_bwd(qkv, out, dout, lse, s: BlockSpec, seq: SeqInfo) -> torch.Tensor:
-    T = qkv.shape[0]
-    lo, hi = seq.bounds()
-    dqkv = torch.empty_like(qkv)
-    delta = torch.empty(s.n_q, T, device=qkv.device, dtype=torch.float32)
-    ws = None
-    if s.n_q > s.n_kv and ((T + 127) // 128) * s.n_kv < 2 * _sm_count():
-        ws = torch.empty(2 * s.n_q * T * s.head_dim, device=qkv.device, dtype=torch.float32)
-    nv.call("mmt_attn_bwd", qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), delta.data_ptr(),
-            dqkv.data_ptr(), lo.data_ptr(), hi.data_ptr(), T, s.n_q, s.n_kv, s.head_dim, qkv.stride(0), int(s.causal),
-            s.scale, nv.ptr(ws), nv.stream())
-    return dqkv
+    return attn_bwd(qkv, out, dout, lse, s.n_q, s.n_kv, s.head_dim, seq, s.causal, s.scale)
 
 
 def _swiglu_fwd(gu: torch.Tensor) -> torch.Tensor:
@@ -128,7 +112,7 @@ def _linear_bwd(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, b) -> torch.
 # --------------------------------------------------------------------------------------
 # Native calls: csrc/block.cu takes one array of 64-bit words (addresses, sizes, flags) in this order
 # --------------------------------------------------------------------------------------
-_N_WORDS = 10 + 6 + 10 + 8 + 10 + 1 + 2 + 4 + 3 + 1
+_N_WORDS = 10 + 6 + 10 + 10 + 10 + 1 + 2 + 4 + 3 + 1
 _Words = ctypes.c_int64 * _N_WORDS
 nv.declare("mmt_block_words", nv.c_int, [])
 nv.declare("mmt_block_fwd", nv.c_int, [nv._P, nv.c_float, nv.c_float, nv._P])
@@ -162,10 +146,12 @@ def _dense(t):
 
 def _front_words(x, y: int, P, cos, sin, seq, s: BlockSpec, act: dict, inter: int) -> list[int]:
     lo, hi = seq.bounds()
+    packs = seq.packs()
     T, C = x.shape
     return [0 if p is None else p.data_ptr() for p in P] + [
         x.data_ptr(), y, cos.data_ptr(), sin.data_ptr(), lo.data_ptr(), hi.data_ptr(), *[act[k] for k in _ACT],
-        T, C, s.n_q, s.n_kv, s.head_dim, s.rope_heads, inter, int(s.causal)]
+        T, C, s.n_q, s.n_kv, s.head_dim, s.rope_heads, inter, int(s.causal),
+        0 if packs is None else packs.data_ptr(), 0 if packs is None else packs.shape[0]]
 
 
 def _native_call(name: str, words, *args) -> None:
@@ -235,8 +221,7 @@ class _LocalBlockFn(torch.autograd.Function):
                 fresh.append((p, mg, g))
                 grads.append(g.data_ptr())
         parts = max(nv.lib().mmt_rmsnorm_bwd_parts(T) * C, nv.lib().mmt_colsum_parts(T) * max(2 * inter, qw, C))
-        # GQA with few KV tiles: one dK/dV CTA per q head needs an fp32 partial-sum workspace
-        split = s.n_q > s.n_kv and ((T + 127) // 128) * s.n_kv < 2 * _sm_count()
+        split = split_heads(T, s.n_q, s.n_kv)
         dx = torch.empty_like(x)
         scratch, addr = _carve([4 * T * inter, 2 * T * max(inter, qw), 2 * T * max(C, aw), 2 * T * C, 4 * s.n_q * T,
                                 8 * s.n_q * T * s.head_dim if split else 0, 4 * parts], dev)

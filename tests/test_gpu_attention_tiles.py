@@ -9,6 +9,15 @@ TOL = 2.5e-2
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("cu", [[0, 2], [0, 128], [0, 127, 128, 256], [0, 1, 129], [0, 64, 128, 160, 288, 289],
+                                [0, 65, 130, 195], [0, 100, 200, 200, 264, 300]])
+@pytest.mark.parametrize("heads,dim,causal", [((3, 3), 80, False), ((4, 4), 128, True), ((6, 2), 128, True)])
+def test_short_sequences(cu, heads, dim, causal):
+    errs = _run(cu, *heads, dim, causal)
+    assert max(errs) < TOL, errs
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("cu", [[0, 129], [0, 257], [0, 130, 385], [0, 256, 512], [0, 200, 230, 700], [0, 384, 385, 640]])
 @pytest.mark.parametrize("heads,dim,causal", [((3, 3), 80, False), ((6, 2), 128, True)])
 def test_query_tile_pairs(cu, heads, dim, causal):
@@ -31,3 +40,11 @@ def test_growing_scores_rescale():
     q, k, v = (t.float().reshape(T, 1, d) for t in qkv.split(d, dim=1))
     ref = F.attention_reference(q, k, v, [0, T], False, 1.0 / math.sqrt(d)).reshape(T, d)
     assert ((out.float() - ref).abs().max() / ref.abs().max()).item() < TOL
+
+
+def test_packs_cover_all_rows_once():
+    from multimodal_training_b200.ops.attention import pack_sequences
+    for cu in ([0, 64, 128, 192], [0, 1, 2, 130], [0, 128, 256], [0, 100, 100, 200, 230], [0, 7]):
+        packs = pack_sequences(cu, 128)
+        assert [r for a, n in packs for r in range(a, a + n)] == list(range(cu[-1]))
+        assert all(0 < n <= 128 and a in cu and a + n in cu for a, n in packs)
