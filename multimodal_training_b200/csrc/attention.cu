@@ -70,7 +70,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
   uint64_t* pv_done = bars + 14;    // [2] per tile
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   constexpr int X2 = 64;
 
   if (threadIdx.x == 0) {
@@ -94,7 +94,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   grid_dependency_sync();
   // non-causal: the CTAs that run together share a head, so its K and V stay in L2 however long the sequence;
   // causal: the last query tiles see the most KV blocks and are started first, over all heads (longest work first)
@@ -118,32 +118,38 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
       last[w] = (hi - kv_base + BKV - 1) / BKV;
     }
   }
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    first[w] = warp_uniform(first[w]);
+    last[w] = warp_uniform(last[w]);
+  }
+  kv_base = warp_uniform(kv_base);
   const int n_blocks = max(last[0], last[1]);
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      auto load = [&](uint8_t* dst, uint64_t* bar, int x, int y) {
+    auto load = [&](uint8_t* dst, uint64_t* bar, int x, int y) {
+      if (elect_one()) {
         mbar_expect_tx(bar, 2 * CHUNK);
         tma_load_2d(dst, &tm, bar, x, y);
         tma_load_2d(dst + CHUNK, &tm, bar, x + X2, y);
-      };
-      bool ok = true;
-      if (last[0] > first[0]) load(sQ, &q_full[0], xq, q0[0]);
-      for (int j = 0; j < n_blocks && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t free_parity = (uint32_t)(((j >> 1) & 1) ^ 1);
-        const int r0 = kv_base + j * BKV;
-        if (!mbar_wait(&k_empty[st], free_parity, p.ew, 410)) { ok = false; break; }
-        load(sK + st * 2 * CHUNK, &k_full[st], xk, r0);
-        if (j == 0 && last[1] > first[1]) load(sQ + 2 * CHUNK, &q_full[1], xq, q0[1]);
-        if (!mbar_wait(&v_empty[st], free_parity, p.ew, 411)) { ok = false; break; }
-        load(sV + st * 2 * CHUNK, &v_full[st], xv, r0);
       }
+      __syncwarp();
+    };
+    if (last[0] > first[0]) load(sQ, &q_full[0], xq, q0[0]);
+    for (int j = 0; j < n_blocks; ++j) {
+      const int st = j & 1;
+      const uint32_t free_parity = (uint32_t)(((j >> 1) & 1) ^ 1);
+      const int r0 = kv_base + j * BKV;
+      if (!mbar_wait_warp(&k_empty[st], free_parity, p.ew, 410)) break;
+      load(sK + st * 2 * CHUNK, &k_full[st], xk, r0);
+      if (j == 0 && last[1] > first[1]) load(sQ + 2 * CHUNK, &q_full[1], xq, q0[1]);
+      if (!mbar_wait_warp(&v_empty[st], free_parity, p.ew, 411)) break;
+      load(sV + st * 2 * CHUNK, &v_full[st], xv, r0);
     }
   } else if (warp == 9) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    {
       const uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
       const uint32_t idesc_pv = make_idesc_bf16(BQ, DIM, 0, 1);
       const uint32_t hi = smem_desc_hi(1024);
@@ -154,6 +160,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
       auto issue_s = [&](int w, int j) {
         const uint32_t d = tmem_base + (uint32_t)(w * 128);
         const uint32_t a = q_lo + (uint32_t)w * kPair, b = k_lo + (uint32_t)(j & 1) * kPair;
+        if (!elect_one()) return;
 #pragma unroll
         for (int k = 0; k < DIM / 16; ++k) {
           const uint32_t off = (uint32_t)(((k >> 2) * CHUNK + (k & 3) * 32) >> 4);
@@ -164,41 +171,48 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
       auto sees = [&](int w, int j) { return j >= first[w] && j < last[w]; };
       int seen[2] = {0, 0};                             // blocks of tile w whose P has been consumed
       bool ok = true;
-      if (n_blocks > 0) ok = mbar_wait(&k_full[0], 0, p.ew, 511);
+      if (n_blocks > 0) ok = mbar_wait_warp(&k_full[0], 0, p.ew, 511);
       for (int w = 0; w < 2 && ok; ++w) {
         if (!sees(w, 0)) continue;
-        ok = mbar_wait(&q_full[w], 0, p.ew, 510);
+        ok = mbar_wait_warp(&q_full[w], 0, p.ew, 510);
         if (ok) issue_s(w, 0);
+        __syncwarp();
       }
-      if (ok && n_blocks > 0) tc_commit(&k_empty[0]);
+      if (ok && n_blocks > 0 && elect_one()) tc_commit(&k_empty[0]);
       for (int j = 0; j < n_blocks && ok; ++j) {
         const int nx = j + 1;
         bool have_k = false, have_v = false;
         for (int w = 0; w < 2 && ok; ++w) {
           if (sees(w, j)) {
-            if (!have_v && !mbar_wait(&v_full[j & 1], (j >> 1) & 1, p.ew, 513)) { ok = false; break; }
+            if (!have_v && !mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, p.ew, 513)) { ok = false; break; }
             have_v = true;
-            if (!mbar_wait(&p_full[w], seen[w] & 1, p.ew, 512)) { ok = false; break; }
+            if (!mbar_wait_warp(&p_full[w], seen[w] & 1, p.ew, 512)) { ok = false; break; }
             tc_fence_after();
             const uint32_t d = tmem_base + 256u + (uint32_t)(w * 128);
             const uint32_t a = tmem_base + (uint32_t)(w * 128);
             const uint32_t b = v_lo + (uint32_t)(j & 1) * kPair;
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BKV / 16; ++k)
-              tc_mma_ts(d, a + (uint32_t)(k * 8), smem_desc_join(hi, b + (uint32_t)(k * (2048 >> 4))), idesc_pv,
-                        (seen[w] | k) != 0);
+              for (int k = 0; k < BKV / 16; ++k)
+                tc_mma_ts(d, a + (uint32_t)(k * 8), smem_desc_join(hi, b + (uint32_t)(k * (2048 >> 4))), idesc_pv,
+                          (seen[w] | k) != 0);
+              if (j == last[w] - 1) tc_commit(&pv_done[w]);
+            }
+            __syncwarp();
             ++seen[w];
-            if (j == last[w] - 1) tc_commit(&pv_done[w]);
           }
-          if (w == 1) tc_commit(&v_empty[j & 1]);
+          if (w == 1 && elect_one()) tc_commit(&v_empty[j & 1]);
+          __syncwarp();
           if (sees(w, nx)) {
-            if (!have_k && !mbar_wait(&k_full[nx & 1], (nx >> 1) & 1, p.ew, 514)) { ok = false; break; }
+            if (!have_k && !mbar_wait_warp(&k_full[nx & 1], (nx >> 1) & 1, p.ew, 514)) { ok = false; break; }
             have_k = true;
-            if (nx == first[w] && !mbar_wait(&q_full[w], 0, p.ew, 515)) { ok = false; break; }
+            if (nx == first[w] && !mbar_wait_warp(&q_full[w], 0, p.ew, 515)) { ok = false; break; }
             issue_s(w, nx);
+            __syncwarp();
           }
         }
-        if (ok && nx < n_blocks) tc_commit(&k_empty[nx & 1]);
+        if (ok && nx < n_blocks && elect_one()) tc_commit(&k_empty[nx & 1]);
+        __syncwarp();
       }
     }
   } else {

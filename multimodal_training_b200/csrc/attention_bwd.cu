@@ -116,7 +116,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   uint64_t* done = row_full + kRowBufs;      // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm_kv);
@@ -142,7 +142,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   grid_dependency_sync();
   const int kv0 = blockIdx.x * BKV;
   const bool split = p.ws_dk != nullptr;
@@ -153,37 +153,42 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   const int kv_last = min(kv0 + BKV, p.T) - 1;
   const int q_lo = p.causal ? kv0 : p.seq_lo[kv0];
   const int q_hi = p.seq_hi[kv_last];
-  const int n_qb = (q_hi - q_lo + BQ2 - 1) / BQ2;
+  const int n_qb = warp_uniform((q_hi - q_lo + BQ2 - 1) / BQ2);
   const int n_iter = n_qb * group;
   const int xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
   const uint32_t t_dv = tmem_base + 256, t_dk = tmem_base + 384;
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 4 * CHUNK);
       tma_load_2d(sK, &tm_kv, kv_full, xk, kv0);
       tma_load_2d(sK + CHUNK, &tm_kv, kv_full, xk + 64, kv0);
       tma_load_2d(sV, &tm_kv, kv_full, xv, kv0);
       tma_load_2d(sV + CHUNK, &tm_kv, kv_full, xv + 64, kv0);
-      for (int it = 0; it < n_iter; ++it) {
-        const int g = it / n_qb, i = it % n_qb;
-        const int head = head0 + g;
-        const int r0 = q_lo + i * BQ2;
-        const int r = it % kRing;
-        if (!mbar_wait(&slot_free[r], ((it / kRing) & 1) ^ 1, p.ew, 730)) break;
-        uint8_t* sQ = sRing + (size_t)r * 4 * QBOX;
-        uint8_t* sDO = sQ + 2 * QBOX;
+    }
+    __syncwarp();
+    int head = head0, i = 0;
+    const int q_first = warp_uniform(q_lo);
+    for (int it = 0; it < n_iter; ++it) {
+      const int r0 = q_first + i * BQ2;
+      const int r = it % kRing;
+      if (!mbar_wait_warp(&slot_free[r], ((it / kRing) & 1) ^ 1, p.ew, 730)) break;
+      uint8_t* sQ = sRing + (size_t)r * 4 * QBOX;
+      uint8_t* sDO = sQ + 2 * QBOX;
+      if (elect_one()) {
         mbar_expect_tx(&slot_full[r], 4 * QBOX);
         tma_load_2d(sQ, &tm_q64, &slot_full[r], head * DIM, r0);
         tma_load_2d(sQ + QBOX, &tm_q64, &slot_full[r], head * DIM + 64, r0);
         tma_load_2d(sDO, &tm_do64, &slot_full[r], head * DIM, r0);
         tma_load_2d(sDO + QBOX, &tm_do64, &slot_full[r], head * DIM + 64, r0);
       }
+      __syncwarp();
+      if (++i == n_qb) { i = 0; ++head; }
     }
   } else if (warp == 9) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    {
       const uint32_t idesc_1 = make_idesc_bf16(BKV, BQ2, 0, 0);     // S^T, dP^T: M = 128 kv rows, N = 64 queries
       const uint32_t idesc_2 = make_idesc_bf16(BKV, DIM, 0, 1);     // dV, dK: A from tensor memory, B MN-major
       const uint32_t hi = smem_desc_hi(1024);
@@ -193,6 +198,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
       auto mma2 = [&](int j) {
         const uint32_t st = tmem_base + (uint32_t)((j & 1) * 128);
         const uint32_t slot = (uint32_t)(j % kRing) * ((4 * QBOX) >> 4);
+        if (!elect_one()) return;
 #pragma unroll
         for (int k = 0; k < BQ2 / 16; ++k) {
           // dV += P^T dO, dK += dS^T Q
@@ -203,36 +209,42 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
         }
         tc_commit(&slot_free[j % kRing]);
       };
-      bool ok = mbar_wait(kv_full, 0, p.ew, 740);
+      bool ok = mbar_wait_warp(kv_full, 0, p.ew, 740);
       for (int it = 0; it < n_iter && ok; ++it) {
         const int r = it % kRing;
-        if (!mbar_wait(&slot_full[r], (it / kRing) & 1, p.ew, 741)) { ok = false; break; }
+        if (!mbar_wait_warp(&slot_full[r], (it / kRing) & 1, p.ew, 741)) { ok = false; break; }
         const uint32_t st = tmem_base + (uint32_t)((it & 1) * 128);
         const uint32_t slot = (uint32_t)r * ((4 * QBOX) >> 4);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < DIM / 16; ++k) {
-          const uint32_t a_off = (uint32_t)(((k >> 2) * CHUNK + (k & 3) * 32) >> 4);
-          const uint32_t b_off = (uint32_t)(((k >> 2) * QBOX + (k & 3) * 32) >> 4);
-          tc_mma_ss(st, smem_desc_join(hi, k_lo + a_off), smem_desc_join(hi, ring_k + slot + b_off), idesc_1, k != 0);
-          tc_mma_ss(st + 64u, smem_desc_join(hi, v_lo + a_off), smem_desc_join(hi, ring_k + slot + ((2 * QBOX) >> 4) + b_off),
-                    idesc_1, k != 0);
+          for (int k = 0; k < DIM / 16; ++k) {
+            const uint32_t a_off = (uint32_t)(((k >> 2) * CHUNK + (k & 3) * 32) >> 4);
+            const uint32_t b_off = (uint32_t)(((k >> 2) * QBOX + (k & 3) * 32) >> 4);
+            tc_mma_ss(st, smem_desc_join(hi, k_lo + a_off), smem_desc_join(hi, ring_k + slot + b_off), idesc_1, k != 0);
+            tc_mma_ss(st + 64u, smem_desc_join(hi, v_lo + a_off), smem_desc_join(hi, ring_k + slot + ((2 * QBOX) >> 4) + b_off),
+                      idesc_1, k != 0);
+          }
+          tc_commit(&s_full[it & 1]);
         }
-        tc_commit(&s_full[it & 1]);
+        __syncwarp();
         if (it > 0) {
           const int j = it - 1;
-          if (!mbar_wait(&pds_full[j & 1], (j >> 1) & 1, p.ew, 742)) { ok = false; break; }
+          if (!mbar_wait_warp(&pds_full[j & 1], (j >> 1) & 1, p.ew, 742)) { ok = false; break; }
           tc_fence_after();
           mma2(j);
+          __syncwarp();
         }
       }
       if (ok && n_iter > 0) {
         const int j = n_iter - 1;
-        if (mbar_wait(&pds_full[j & 1], (j >> 1) & 1, p.ew, 743)) {
+        if (mbar_wait_warp(&pds_full[j & 1], (j >> 1) & 1, p.ew, 743)) {
           tc_fence_after();
           mma2(j);
+          __syncwarp();
         }
       }
-      tc_commit(done);
+      if (elect_one()) tc_commit(done);
+      __syncwarp();
     }
   } else {
     // ------------------------------ softmax warps (8) + epilogue ------------------------------
@@ -414,7 +426,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint64_t* done = ds_full + 2;              // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm_q);
@@ -439,7 +451,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   grid_dependency_sync();
   // causal: the last query tiles see the most KV blocks and are started first
   const int q0 = (p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x) * BQ;
@@ -448,32 +460,37 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int q_last = min(q0 + BQ, p.T) - 1;
   const int kv_lo = p.seq_lo[q0];
   const int kv_hi = p.causal ? min(p.seq_hi[q_last], q_last + 1) : p.seq_hi[q_last];
-  const int n_iter = (kv_hi - kv_lo + BQ2 - 1) / BQ2;
+  const int n_iter = warp_uniform((kv_hi - kv_lo + BQ2 - 1) / BQ2);
   const int xq = head * DIM, xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
   const uint32_t t_dq = tmem_base + 256;
 
   if (warp == 8) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, 4 * CHUNK);
       tma_load_2d(sQ, &tm_q, q_full, xq, q0);
       tma_load_2d(sQ + CHUNK, &tm_q, q_full, xq + 64, q0);
       tma_load_2d(sDO, &tm_do, q_full, xq, q0);
       tma_load_2d(sDO + CHUNK, &tm_do, q_full, xq + 64, q0);
-      for (int it = 0; it < n_iter; ++it) {
-        const int r0 = kv_lo + it * BQ2;
-        const int r = it % kRing;
-        if (!mbar_wait(&slot_free[r], ((it / kRing) & 1) ^ 1, p.ew, 760)) break;
-        uint8_t* sKb = sRing + (size_t)r * 4 * QBOX;
-        uint8_t* sVb = sKb + 2 * QBOX;
+    }
+    __syncwarp();
+    const int kv_first = warp_uniform(kv_lo);
+    for (int it = 0; it < n_iter; ++it) {
+      const int r0 = kv_first + it * BQ2;
+      const int r = it % kRing;
+      if (!mbar_wait_warp(&slot_free[r], ((it / kRing) & 1) ^ 1, p.ew, 760)) break;
+      uint8_t* sKb = sRing + (size_t)r * 4 * QBOX;
+      uint8_t* sVb = sKb + 2 * QBOX;
+      if (elect_one()) {
         mbar_expect_tx(&slot_full[r], 4 * QBOX);
         tma_load_2d(sKb, &tm_kv64, &slot_full[r], xk, r0);
         tma_load_2d(sKb + QBOX, &tm_kv64, &slot_full[r], xk + 64, r0);
         tma_load_2d(sVb, &tm_kv64, &slot_full[r], xv, r0);
         tma_load_2d(sVb + QBOX, &tm_kv64, &slot_full[r], xv + 64, r0);
       }
+      __syncwarp();
     }
   } else if (warp == 9) {
-    if (lane == 0) {
+    {
       const uint32_t idesc_1 = make_idesc_bf16(BQ, BQ2, 0, 0);      // S, dP: M = 128 queries, N = 64 kv rows
       const uint32_t idesc_2 = make_idesc_bf16(BQ, DIM, 0, 1);      // dQ: A from tensor memory, B = K block MN-major
       const uint32_t hi = smem_desc_hi(1024);
@@ -483,42 +500,49 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       auto mma2 = [&](int j) {
         const uint32_t st = tmem_base + (uint32_t)((j & 1) * 128);
         const uint32_t slot = (uint32_t)(j % kRing) * ((4 * QBOX) >> 4);
+        if (!elect_one()) return;
 #pragma unroll
         for (int k = 0; k < BQ2 / 16; ++k)
           tc_mma_ts(t_dq, st + 64u + (uint32_t)(k * 8), smem_desc_join(hi, ring_mn + slot + (uint32_t)(k * 128)), idesc_2,
                     (j | k) != 0);
         tc_commit(&slot_free[j % kRing]);
       };
-      bool ok = mbar_wait(q_full, 0, p.ew, 770);
+      bool ok = mbar_wait_warp(q_full, 0, p.ew, 770);
       for (int it = 0; it < n_iter && ok; ++it) {
         const int r = it % kRing;
-        if (!mbar_wait(&slot_full[r], (it / kRing) & 1, p.ew, 771)) { ok = false; break; }
+        if (!mbar_wait_warp(&slot_full[r], (it / kRing) & 1, p.ew, 771)) { ok = false; break; }
         const uint32_t st = tmem_base + (uint32_t)((it & 1) * 128);
         const uint32_t slot = (uint32_t)r * ((4 * QBOX) >> 4);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < DIM / 16; ++k) {
-          const uint32_t a_off = (uint32_t)(((k >> 2) * CHUNK + (k & 3) * 32) >> 4);
-          const uint32_t b_off = (uint32_t)(((k >> 2) * QBOX + (k & 3) * 32) >> 4);
-          tc_mma_ss(st, smem_desc_join(hi, q_lo + a_off), smem_desc_join(hi, ring_k + slot + b_off), idesc_1, k != 0);
-          tc_mma_ss(st + 64u, smem_desc_join(hi, do_lo + a_off), smem_desc_join(hi, ring_k + slot + ((2 * QBOX) >> 4) + b_off),
-                    idesc_1, k != 0);
+          for (int k = 0; k < DIM / 16; ++k) {
+            const uint32_t a_off = (uint32_t)(((k >> 2) * CHUNK + (k & 3) * 32) >> 4);
+            const uint32_t b_off = (uint32_t)(((k >> 2) * QBOX + (k & 3) * 32) >> 4);
+            tc_mma_ss(st, smem_desc_join(hi, q_lo + a_off), smem_desc_join(hi, ring_k + slot + b_off), idesc_1, k != 0);
+            tc_mma_ss(st + 64u, smem_desc_join(hi, do_lo + a_off), smem_desc_join(hi, ring_k + slot + ((2 * QBOX) >> 4) + b_off),
+                      idesc_1, k != 0);
+          }
+          tc_commit(&s_full[it & 1]);
         }
-        tc_commit(&s_full[it & 1]);
+        __syncwarp();
         if (it > 0) {
           const int j = it - 1;
-          if (!mbar_wait(&ds_full[j & 1], (j >> 1) & 1, p.ew, 772)) { ok = false; break; }
+          if (!mbar_wait_warp(&ds_full[j & 1], (j >> 1) & 1, p.ew, 772)) { ok = false; break; }
           tc_fence_after();
           mma2(j);
+          __syncwarp();
         }
       }
       if (ok && n_iter > 0) {
         const int j = n_iter - 1;
-        if (mbar_wait(&ds_full[j & 1], (j >> 1) & 1, p.ew, 773)) {
+        if (mbar_wait_warp(&ds_full[j & 1], (j >> 1) & 1, p.ew, 773)) {
           tc_fence_after();
           mma2(j);
+          __syncwarp();
         }
       }
-      tc_commit(done);
+      if (elect_one()) tc_commit(done);
+      __syncwarp();
     }
   } else {
     const int q4 = warp & 3;

@@ -44,7 +44,7 @@ attn_local_fwd_kernel(const __grid_constant__ CUtensorMap tm, const LocalParams 
   uint64_t* p_full = qk_full + 3;
   uint64_t* o_full = qk_full + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(qk_full + 5);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm);
@@ -62,15 +62,15 @@ attn_local_fwd_kernel(const __grid_constant__ CUtensorMap tm, const LocalParams 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t t_s = *tmem_slot, t_o = t_s + 128;      // S (P over its first 64 columns), O
+  const uint32_t t_s = warp_uniform(*tmem_slot), t_o = t_s + 128;      // S (P over its first 64 columns), O
   grid_dependency_sync();
   const int head = (int)blockIdx.x % p.n_q, item = (int)blockIdx.x / p.n_q;
-  const int r0 = lp.items[2 * item], rows = lp.items[2 * item + 1];
+  const int r0 = warp_uniform(lp.items[2 * item]), rows = lp.items[2 * item + 1];
 
   if (warp == 4) {
-    if (lane == 0) {
-      const int kv_head = head / (p.n_q / p.n_kv);
-      const int xq = head * DIM, xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
+    const int kv_head = head / (p.n_q / p.n_kv);
+    const int xq = head * DIM, xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
+    if (elect_one()) {
       mbar_expect_tx(qk_full, 4 * CHUNK);
       tma_load_2d(sQ, &tm, qk_full, xq, r0);
       tma_load_2d(sK, &tm, qk_full, xk, r0);
@@ -79,15 +79,21 @@ attn_local_fwd_kernel(const __grid_constant__ CUtensorMap tm, const LocalParams 
       mbar_expect_tx(v_full, 2 * CHUNK);
       tma_load_2d(sV, &tm, v_full, xv, r0);
       tma_load_2d(sV + CHUNK, &tm, v_full, xv + 64, r0);
-      if (mbar_wait(qk_full, 0, p.ew, 800)) {
-        const uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
+    }
+    __syncwarp();
+    if (mbar_wait_warp(qk_full, 0, p.ew, 800)) {
+      const uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < DIM / 16; ++k)
           tc_mma_ss(t_s, desc_kmajor(smem_u32(sQ), k), desc_kmajor(smem_u32(sK), k), idesc_s, k != 0);
         tc_commit(s_full);
-        if (mbar_wait(v_full, 0, p.ew, 801) && mbar_wait(p_full, 0, p.ew, 802)) {
-          tc_fence_after();
-          const uint32_t idesc_pv = make_idesc_bf16(BQ, DIM, 0, 1);
+      }
+      __syncwarp();
+      if (mbar_wait_warp(v_full, 0, p.ew, 801) && mbar_wait_warp(p_full, 0, p.ew, 802)) {
+        tc_fence_after();
+        const uint32_t idesc_pv = make_idesc_bf16(BQ, DIM, 0, 1);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BKV / 16; ++k)
             tc_mma_ts(t_o, t_s + (uint32_t)(k * 8), desc_mnmajor(smem_u32(sV), k), idesc_pv, k != 0);
@@ -95,6 +101,7 @@ attn_local_fwd_kernel(const __grid_constant__ CUtensorMap tm, const LocalParams 
         }
       }
     }
+    __syncwarp();
   } else {
     const int row = warp * 32 + lane;
     const int qrow = r0 + row;
@@ -212,7 +219,7 @@ attn_local_bwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
   uint64_t* pds_full = qk_full + 3;
   uint64_t* grad_full = qk_full + 4;           // [3]: dV, dK, dQ
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(qk_full + 7);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm);
@@ -231,14 +238,14 @@ attn_local_bwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t t_s = *tmem_slot, t_dp = t_s + 128, t_dq = t_s + 256, t_dk = t_s + 384, t_dv = t_s;
+  const uint32_t t_s = warp_uniform(*tmem_slot), t_dp = t_s + 128, t_dq = t_s + 256, t_dk = t_s + 384, t_dv = t_s;
   grid_dependency_sync();
   const int head = (int)blockIdx.x % p.n_q, item = (int)blockIdx.x / p.n_q;
-  const int r0 = lp.items[2 * item], rows = lp.items[2 * item + 1];
+  const int r0 = warp_uniform(lp.items[2 * item]), rows = lp.items[2 * item + 1];
   const int xq = head * DIM, xk = (p.n_q + head) * DIM, xv = (2 * p.n_q + head) * DIM;
 
   if (warp == 8) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(qk_full, 4 * CHUNK);
       tma_load_2d(sQ, &tm, qk_full, xq, r0);
       tma_load_2d(sK, &tm, qk_full, xk, r0);
@@ -249,23 +256,32 @@ attn_local_bwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
       tma_load_2d(sV, &tm, dov_full, xv, r0);
       tma_load_2d(sDO + CHUNK, &tm_do, dov_full, xq + 64, r0);
       tma_load_2d(sV + CHUNK, &tm, dov_full, xv + 64, r0);
-      const uint32_t q = smem_u32(sQ), k_ = smem_u32(sK), d_o = smem_u32(sDO), v = smem_u32(sV), ds = smem_u32(sDS);
-      const uint32_t idesc_1 = make_idesc_bf16(128, 128, 0, 0);
-      bool ok = mbar_wait(qk_full, 0, p.ew, 820);
-      if (ok) {
+    }
+    __syncwarp();
+    const uint32_t q = smem_u32(sQ), k_ = smem_u32(sK), d_o = smem_u32(sDO), v = smem_u32(sV), ds = smem_u32(sDS);
+    const uint32_t idesc_1 = make_idesc_bf16(128, 128, 0, 0);
+    bool ok = mbar_wait_warp(qk_full, 0, p.ew, 820);
+    if (ok) {
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < DIM / 16; ++k) tc_mma_ss(t_s, desc_kmajor(q, k), desc_kmajor(k_, k), idesc_1, k != 0);
-        ok = mbar_wait(dov_full, 0, p.ew, 821);
       }
-      if (ok) {
+      __syncwarp();
+      ok = mbar_wait_warp(dov_full, 0, p.ew, 821);
+    }
+    if (ok) {
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < DIM / 16; ++k) tc_mma_ss(t_dp, desc_kmajor(d_o, k), desc_kmajor(v, k), idesc_1, k != 0);
         tc_commit(s_full);
-        ok = mbar_wait(pds_full, 0, p.ew, 822);
       }
-      if (ok) {
-        tc_fence_after();
-        const uint32_t idesc_t = make_idesc_bf16(128, DIM, 1, 1), idesc_q = make_idesc_bf16(128, DIM, 0, 1);
+      __syncwarp();
+      ok = mbar_wait_warp(pds_full, 0, p.ew, 822);
+    }
+    if (ok) {
+      tc_fence_after();
+      const uint32_t idesc_t = make_idesc_bf16(128, DIM, 1, 1), idesc_q = make_idesc_bf16(128, DIM, 0, 1);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) tc_mma_ss(t_dv, desc_mnmajor(v, k), desc_mnmajor(d_o, k), idesc_t, k != 0);
         tc_commit(&grad_full[0]);
@@ -276,6 +292,7 @@ attn_local_bwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
         for (int k = 0; k < 8; ++k) tc_mma_ss(t_dq, desc_kmajor(ds, k), desc_mnmajor(k_, k), idesc_q, k != 0);
         tc_commit(&grad_full[2]);
       }
+      __syncwarp();
     }
   } else {
     const int q4 = warp & 3, half = warp >> 2;

@@ -141,6 +141,20 @@ MMT_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, MmtErrorWord* ew, int 
   }
 }
 
+// The same by a whole warp, with one answer.
+MMT_DEVICE bool mbar_wait_warp(uint64_t* bar, uint32_t parity, MmtErrorWord* ew, int where) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, ew, where));
+}
+
+// Warp-uniform values.  The operands of tcgen05.mma and of TMA copies live in uniform registers.  A loop that only one
+// lane runs (`if (lane == 0)`) computes them per thread and moves every word of every descriptor over, one after the
+// other; a loop that the whole warp runs on values the compiler knows to be the same in all lanes keeps them there.
+// So the issuing warps run their loops together and elect a lane for the instructions alone.
+// Measured: 1024 x 1280 x 3840 (128-row tiles, 64-wide k-blocks) 30.5 -> 24.7 us, 4096 x 1280 x 6848 (256-row tiles)
+// 65.6 -> 62.3 us; attention forward and backward of 16384 patches 1.75 -> 1.64 and 7.00 -> 6.28 ms.
+MMT_DEVICE int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+MMT_DEVICE uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // One non-blocking look at an mbarrier phase (true = that phase has completed).
 MMT_DEVICE bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;

@@ -736,7 +736,7 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint64_t* fwd_done = fwd_go + kStages;  // [kStages]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fwd_done + kStages);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform((int)threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   long long clk_c0 = 0;
   unsigned long long clk_t0 = 0;
@@ -771,12 +771,50 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   grid_dependency_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (!p.ag_flags && !p.kf_flags) {
+      // operands in this GPU's memory, complete before the launch: nothing but the ring to wait for.  This loop paces
+      // the main loop of short tiles, so the warp runs it together (warp_uniform, common.cuh)
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      int kcount = 0;
+      WorkItem w;
+      for (int wi = 0; ok && work_item(p, wi, blockIdx.x, gridDim.x, KB, ntiles, w); ++wi) {
+        int tm, tn;
+        tile_coords(p, w.tile, tiles_m, BMT, tm, tn);
+        for (int kb = w.k0; kb < w.k1; ++kb) {
+          if ((MMT_DBG & 1) && kcount++ >= kStages) continue;
+          if (!mbar_wait_warp(&empty[s], ph ^ 1, p.ew, 102)) { ok = false; break; }
+          uint8_t* sA = smem + (size_t)s * C_::STAGE_BYTES;
+          uint8_t* sB = sA + C_::A_BYTES;
+          if (elect_one()) {
+            mbar_expect_tx(&full[s], C_::STAGE_BYTES);
+            if (!p.a_mn) {
+              tma_load_2d(sA, &tmA, &full[s], kb * BK, tm * BMT);      // one box of BMT rows
+            } else {
+#pragma unroll
+              for (int c = 0; c < BMT / 64; ++c) tma_load_2d(sA + c * 8192, &tmA, &full[s], tm * BMT + c * 64, kb * BK);
+            }
+            if (!p.b_mn) {
+              tma_load_2d(sB, &tmB, &full[s], kb * BK, tn * BN);
+            } else {
+#pragma unroll
+              for (int c = 0; c < BN / 64; ++c) tma_load_2d(sB + c * 8192, &tmB, &full[s], tn * BN + c * 64, kb * BK);
+            }
+          }
+          __syncwarp();
+          if (++s == kStages) { s = 0; ph ^= 1; }
+        }
+      }
+      // the last operand tile is on its way: CTAs of the next kernel may become resident (not earlier: from the
+      // start of a GEMM they would sit on the SMs that this grid leaves free for its whole run)
+      if (p.local_only) grid_dependents_launch();
+    } else if (lane == 0) {
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -857,13 +895,10 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           if (++s == kStages) { s = 0; ph ^= 1; }
         }
       }
-      // the last operand tile is on its way: CTAs of the next kernel may become resident (not earlier: from the
-      // start of a GEMM they would sit on the SMs that this grid leaves free for its whole run)
-      if (p.local_only) grid_dependents_launch();
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    {
       const uint32_t idesc = make_idesc_bf16(BM, BN, p.a_mn, p.b_mn);
       // descriptor halves, encoded once: per instruction only the start-address field moves
       const uint32_t a_hi = smem_desc_hi(p.a_mn ? p.mn_sbo : 1024u), b_hi = smem_desc_hi(p.b_mn ? p.mn_sbo : 1024u);
@@ -875,15 +910,13 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       uint32_t ph = 0, acc_ph = 0;   // MT == 1: acc alternates per tile; MT == 2: slots 0/1 are the halves
       bool ok = true;
       int kcount = 0;
-      // The issue loop is kept as short as it can be: this one thread has to hand the tensor core an instruction
-      // every ~128 cycles.  Whether the NEXT ring slot is full is looked up (non-blocking) in the shadow of the
-      // current slot's instructions, so the common case never waits for a barrier round trip.
-      bool ready = false;
+      // The issue loop is kept as short as it can be: a k-block of a 64-column tile occupies the tensor core for some
+      // 130 cycles only.  The warp runs it together (warp_uniform, common.cuh); one lane issues.
       WorkItem w;
       for (int wi = 0; ok && work_item(p, wi, blockIdx.x, gridDim.x, KB, ntiles, w); ++wi) {
         // the accumulator (MT == 1) or both halves (MT == 2) of an earlier tile must have been drained
-        if (!mbar_wait(&tempty[MT == 2 ? 0 : acc], acc_ph ^ 1, p.ew, 200)) { ok = false; break; }
-        if (MT == 2 && !mbar_wait(&tempty[1], acc_ph ^ 1, p.ew, 202)) { ok = false; break; }
+        if (!mbar_wait_warp(&tempty[MT == 2 ? 0 : acc], acc_ph ^ 1, p.ew, 200)) { ok = false; break; }
+        if (MT == 2 && !mbar_wait_warp(&tempty[1], acc_ph ^ 1, p.ew, 202)) { ok = false; break; }
         tc_fence_after();
         int fwd_tn = -1;                 // >= 0: this tile forwards its k-blocks kb % fwd_split == fwd_tn
         if (p.fwd_peers > 0) {
@@ -894,37 +927,43 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const uint32_t d0 = tmem_base + (uint32_t)((MT == 2 ? 0 : acc) * BN);
         for (int kb = 0; kb < w.k1 - w.k0; ++kb) {      // kb counts from the start of this run: a fresh accumulator
           const bool skip = (MMT_DBG & 1) && kcount++ >= kStages;
-          if (!ready && !skip && !mbar_wait(&full[s], ph, p.ew, 201)) { ok = false; break; }
+          if (!skip && !mbar_wait_warp(&full[s], ph, p.ew, 201)) { ok = false; break; }
           const uint32_t so = (uint32_t)s * (C_::STAGE_BYTES >> 4);
           int sn = s + 1;
           uint32_t phn = ph;
           if (sn == kStages) { sn = 0; phn ^= 1; }
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t bdesc = smem_desc_join(b_hi, b_lo0 + so + (uint32_t)k * b_k);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              const uint64_t bdesc = smem_desc_join(b_hi, b_lo0 + so + (uint32_t)k * b_k);
 #pragma unroll
-            for (int h = 0; h < MT; ++h) {
-              // half h: 128 rows further (K-major) or two 64-column chunks further (MN-major)
-              const uint64_t adesc =
-                  smem_desc_join(a_hi, a_lo0 + so + (uint32_t)h * ((BM * BK * 2) >> 4) + (uint32_t)k * a_k);
-              tc_mma_ss(d0 + (uint32_t)(h * BN), adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+              for (int h = 0; h < MT; ++h) {
+                // half h: 128 rows further (K-major) or two 64-column chunks further (MN-major)
+                const uint64_t adesc =
+                    smem_desc_join(a_hi, a_lo0 + so + (uint32_t)h * ((BM * BK * 2) >> 4) + (uint32_t)k * a_k);
+                tc_mma_ss(d0 + (uint32_t)(h * BN), adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+              }
             }
-            if (k == 0) ready = mbar_test(&full[sn], phn);
+            // the stage has landed: the forwarder may send it on
+            if (fwd_tn >= 0 && (w.k0 + kb) % p.fwd_split == fwd_tn) mbar_arrive(&fwd_go[s]);
+            if (!(MMT_DBG & 2)) tc_commit(&empty[s]);
           }
-          // the stage has landed: the forwarder may send it on
-          if (fwd_tn >= 0 && (w.k0 + kb) % p.fwd_split == fwd_tn) mbar_arrive(&fwd_go[s]);
-          if (!(MMT_DBG & 2)) tc_commit(&empty[s]);
+          __syncwarp();
           s = sn;
           ph = phn;
         }
         if (!ok) break;
         if (MT == 1) {
-          tc_commit(&tfull[acc]);
+          if (elect_one()) tc_commit(&tfull[acc]);
+          __syncwarp();
           acc ^= 1;
           if (acc == 0) acc_ph ^= 1;
         } else {
-          tc_commit(&tfull[0]);
-          tc_commit(&tfull[1]);
+          if (elect_one()) {
+            tc_commit(&tfull[0]);
+            tc_commit(&tfull[1]);
+          }
+          __syncwarp();
           acc_ph ^= 1;
         }
       }
