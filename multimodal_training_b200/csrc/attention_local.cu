@@ -328,7 +328,7 @@ attn_local_bwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
       }
     }
     sDelta[half * 128 + row] = part;
-    pair_bar_sync(q4);
+    quadrant_bar_sync<2>(q4);
     const float delta = part + sDelta[(half ^ 1) * 128 + row];
     const float sl2 = p.scale * LOG2E;
     const float2 sl2_2 = make_float2(sl2, sl2), scale_2 = make_float2(p.scale, p.scale);
