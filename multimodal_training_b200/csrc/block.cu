@@ -1,6 +1,6 @@
 // One transformer block per call: the host side of ops/blocks.py in native code.
 //
-// A block is 9 launches forward and up to 31 backward.  Issued one by one from Python (a ctypes call with up to 21
+// A block is 9 launches forward and up to 26 backward.  Issued one by one from Python (a ctypes call with up to 21
 // arguments, an output allocation and several tensor lookups each) a launch costs 15-20 us of host time, which is more
 // than many of these kernels run: at 256 patches the vision encoder took 6.3 ms for 3.6 ms of device work.  Here a
 // block is one call with one array of addresses.
@@ -12,12 +12,15 @@
 
 extern "C" {
 int mmt_rmsnorm_fwd(const void*, const void*, void*, float*, long, int, float, void*);
-int mmt_rmsnorm_bwd_add(const void*, const void*, const void*, const float*, const void*, void*, void*, float*, long,
-                        int, int, void*);
+int mmt_rmsnorm_bwd_parts(long);
+int mmt_rmsnorm_bwd_add_partial(const void*, const void*, const void*, const float*, const void*, void*, float*, long, int,
+                                int*, void*);
 int mmt_rope(void*, const float*, const float*, long, int, int, long, int, void*);
 int mmt_swiglu_fwd(const void*, void*, long, int, void*);
 int mmt_swiglu_bwd(const void*, const void*, void*, long, int, void*);
-int mmt_colsum(const void*, void*, float*, long, int, long, int, void*);
+int mmt_colsum_parts(long);
+int mmt_colsum_partial(const void*, float*, long, int, long, void*);
+int mmt_reduce_partials(const MmtReduceSegment*, int, void*);
 int mmt_gemm_bf16(const void*, const void*, void*, const void*, const void*, int, int, int, int, int, int, int, int, int,
                   int, int, int, float, int, void*);
 int mmt_attn_fwd(const void*, void*, float*, const int*, const int*, long, int, int, int, long, int, float, void*);
@@ -47,7 +50,7 @@ struct BlockArgs {
   int64_t accumulate;            // bit i: add to g[i]
   uint64_t dy, dx;
   uint64_t dgu, big, mid, dx1;   // scratch: [T, 2 inter], [T, max(inter, qkv width)], [T, max(C, n_q dim)], [T, C]
-  uint64_t delta, ws, part;      // attention scratch (ws may be 0); fp32 partial sums of norms and biases
+  uint64_t delta, ws, part;      // attention scratch (ws may be 0); fp32 partial sums of norms and biases, one after the other
   int64_t launches;              // out: kernels launched
 };
 static_assert(sizeof(BlockArgs) % 8 == 0, "an array of 64-bit words");
@@ -56,6 +59,16 @@ struct Issue {
   BlockArgs& b;
   void* st;
   int rc = 0;
+  // partial sums of biases and norm weights, finished by one launch at the end of backward
+  MmtReduceSegment sums[MMT_MAX_REDUCE_SEGMENTS];
+  int n_sums = 0;
+  long part_used = 0;            // floats of b.part in use
+  float* partial_rows(int wi, int parts, long cols) {
+    float* at = f(b.part) + part_used;
+    part_used += (long)parts * cols;
+    sums[n_sums++] = MmtReduceSegment{at, p(b.g[wi]), parts, (int)cols, acc(wi)};
+    return at;
+  }
   void* p(uint64_t v) const { return reinterpret_cast<void*>(v); }
   float* f(uint64_t v) const { return reinterpret_cast<float*>(v); }
   const int* i(uint64_t v) const { return reinterpret_cast<const int*>(v); }
@@ -76,7 +89,7 @@ struct Issue {
     done(mmt_gemm_bf16(p(dy), p(x), p(b.g[wi]), nullptr, nullptr, (int)n, (int)k, (int)b.T, (int)n, (int)k, (int)k, 0, 1,
                        1, 0, acc(wi), 0, 1.f, 0, st), 1);
     if (!rc && b.w[wi + 1])
-      done(mmt_colsum(p(dy), p(b.g[wi + 1]), f(b.part), b.T, (int)n, n, acc(wi + 1), st), 2);
+      done(mmt_colsum_partial(p(dy), partial_rows(wi + 1, mmt_colsum_parts(b.T), n), b.T, (int)n, n, st), 1);
     if (rc) return;
     done(mmt_gemm_bf16(p(dy), p(b.w[wi]), p(dx), nullptr, nullptr, (int)b.T, (int)k, (int)n, (int)n, (int)k, (int)k, 0, 0,
                        1, 0, 0, 0, 1.f, 0, st), 1);
@@ -87,8 +100,9 @@ struct Issue {
   }
   void norm_bwd(uint64_t dy, uint64_t x, int wi, uint64_t rstd, uint64_t extra, uint64_t dx) {
     if (rc) return;
-    done(mmt_rmsnorm_bwd_add(p(dy), p(x), p(b.w[wi]), f(rstd), p(extra), p(dx), p(b.g[wi]), f(b.part), b.T, (int)b.C,
-                             acc(wi), st), 2);
+    float* at = partial_rows(wi, mmt_rmsnorm_bwd_parts(b.T), b.C);
+    done(mmt_rmsnorm_bwd_add_partial(p(dy), p(x), p(b.w[wi]), f(rstd), p(extra), p(dx), at, b.T, (int)b.C,
+                                     &sums[n_sums - 1].parts, st), 1);
   }
   void rope(uint64_t t, int inverse) {
     if (rc) return;
@@ -173,6 +187,7 @@ int mmt_block_bwd(int64_t* words, float scale, void* stream) {
   s.rope(b.big, 1);
   s.linear_bwd(b.big, b.h1, QKV_W, b.mid, qw, b.C);
   s.norm_bwd(b.mid, b.x, LN1, b.rstd1, b.dx1, b.dx);
+  if (!s.rc) s.done(mmt_reduce_partials(s.sums, s.n_sums, stream), 1);
   return s.rc;
 }
 

@@ -276,11 +276,21 @@ __global__ void __launch_bounds__(kNormThreads, VEC <= 2 ? 2 : 1) rmsnorm_bwd_ke
 
 // out[c] (+)= sum_p partial[p, c]; out is bf16.  Block (32 columns, 8 part lanes): the parts are summed by eight
 // lanes with independent loads and combined in a fixed order, so the result does not depend on scheduling.
-__global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, bf16* __restrict__ out,
-                                                              int parts, int cols, int accumulate) {
+// A launch takes several such sums (column blocks of segment after segment): a transformer block has six, of 2 to 5 us
+// each, most of which is launch and one pass of latency.
+struct ReduceSegments {
+  MmtReduceSegment seg[MMT_MAX_REDUCE_SEGMENTS];
+  int n;
+};
+__global__ void __launch_bounds__(256) reduce_partials_kernel(const ReduceSegments r) {
   grid_dependency_sync();
   __shared__ float red[8][33];
-  const int c = blockIdx.x * 32 + threadIdx.x;
+  int block = (int)blockIdx.x, k = 0;
+  while (k + 1 < r.n && block >= (r.seg[k].cols + 31) / 32) block -= (r.seg[k++].cols + 31) / 32;
+  const float* partial = r.seg[k].partial;
+  bf16* out = reinterpret_cast<bf16*>(r.seg[k].out);
+  const int parts = r.seg[k].parts, cols = r.seg[k].cols;
+  const int c = block * 32 + threadIdx.x;
   float s = 0.f;
   if (c < cols) {
 #pragma unroll 4
@@ -291,8 +301,8 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
   if (threadIdx.y == 0 && c < cols) {
     float t = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
-    if (accumulate) t += __bfloat162float(out[c]);
+    for (int q = 0; q < 8; ++q) t += red[q][threadIdx.x];
+    if (r.seg[k].accumulate) t += __bfloat162float(out[c]);
     out[c] = __float2bfloat16(t);
   }
 }
@@ -742,10 +752,24 @@ int mmt_rmsnorm_bwd_parts(long rows) {
   return (int)(rows < cap ? (rows > 0 ? rows : 1) : cap);
 }
 
+// Sums of several sets of partial rows in one launch.
+int mmt_reduce_partials(const MmtReduceSegment* segments, int n, void* stream) {
+  if (n < 0 || n > MMT_MAX_REDUCE_SEGMENTS) return -2;
+  ReduceSegments r = {};
+  unsigned blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    if (segments[i].cols <= 0) continue;
+    r.seg[r.n++] = segments[i];
+    blocks += (unsigned)(segments[i].cols + 31) / 32;
+  }
+  if (blocks == 0) return 0;
+  return (int)launch_dependent(reduce_partials_kernel, blocks, dim3(32, 8), 0, ST(stream), r);
+}
+
 static void launch_reduce_partials(const float* scratch, void* out, int parts, int cols, int accumulate,
                                    void* stream) {
-  launch_dependent(reduce_partials_kernel, (cols + 31) / 32, dim3(32, 8), 0, ST(stream),
-                     scratch, BF(out), parts, cols, accumulate);
+  const MmtReduceSegment s = {scratch, out, parts, cols, accumulate};
+  mmt_reduce_partials(&s, 1, stream);
 }
 
 // Launches the backward kernel on at most `max_parts` CTAs; returns the number of partial rows it wrote.
@@ -778,6 +802,15 @@ int mmt_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* r
   const int parts = launch_rmsnorm_bwd(dy, x, w, rstd, nullptr, dx, scratch, rows, cols, mmt_rmsnorm_bwd_parts(rows),
                                        stream);
   launch_reduce_partials(scratch, dw, parts, cols, accumulate_dw, stream);
+  return (int)cudaGetLastError();
+}
+
+// First stage of mmt_rmsnorm_bwd_add: dx, and *parts rows of partial sums of dw in scratch.
+int mmt_rmsnorm_bwd_add_partial(const void* dy, const void* x, const void* w, const float* rstd, const void* extra,
+                                void* dx, float* scratch, long rows, int cols, int* parts, void* stream) {
+  if (cols % 8 || cols > 8 * kNormThreads * kNormVec) return -2;
+  if (rows <= 0 || rows > 0x7fffffffL) return -5;     // the kernel indexes rows with 32-bit integers
+  *parts = launch_rmsnorm_bwd(dy, x, w, rstd, extra, dx, scratch, rows, cols, mmt_rmsnorm_bwd_parts(rows), stream);
   return (int)cudaGetLastError();
 }
 
@@ -876,14 +909,18 @@ int mmt_colsum_parts(long rows) {
   const int cap = 64;
   return (int)(p < 1 ? 1 : (p > cap ? cap : p));
 }
+// First stage of mmt_colsum: mmt_colsum_parts(rows) rows of partial sums in scratch.
+int mmt_colsum_partial(const void* x, float* scratch, long rows, int cols, long ld, void* stream) {
+  if (cols % 8 || ld % 8) return -2;
+  const dim3 grid((cols + 255) / 256, mmt_colsum_parts(rows));
+  return (int)launch_dependent(colsum_partial_kernel, grid, dim3(32, 8), 0, ST(stream), CBF(x), scratch, rows, cols, ld);
+}
 // out[c] (+)= sum_r x[r,c]; scratch fp32 [parts, cols].
 int mmt_colsum(const void* x, void* out, float* scratch, long rows, int cols, long ld, int accumulate, void* stream) {
   if (cols % 8 || ld % 8) return -2;
-  const int parts = mmt_colsum_parts(rows);
-  dim3 grid((cols + 255) / 256, parts), block(32, 8);
-  launch_dependent(colsum_partial_kernel, grid, block, 0, ST(stream),
-                     CBF(x), scratch, rows, cols, ld);
-  launch_reduce_partials(scratch, out, parts, cols, accumulate, stream);
+  const int rc = mmt_colsum_partial(x, scratch, rows, cols, ld, stream);
+  if (rc) return rc;
+  launch_reduce_partials(scratch, out, mmt_colsum_parts(rows), cols, accumulate, stream);
   return (int)cudaGetLastError();
 }
 

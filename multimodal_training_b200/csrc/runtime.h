@@ -34,6 +34,14 @@ cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// One sum of partial rows: out[c] (+)= sum over parts of partial[part][c] (fp32 -> bf16).
+struct MmtReduceSegment {
+  const float* partial;
+  void* out;
+  int parts, cols, accumulate;
+};
+#define MMT_MAX_REDUCE_SEGMENTS 6
+
 extern "C" {
 // Copies the error word to out[4] = {code, where, block, aux}; synchronises the device.
 int mmt_get_error(int* out);

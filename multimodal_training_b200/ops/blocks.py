@@ -220,7 +220,8 @@ class _LocalBlockFn(torch.autograd.Function):
                 g = torch.empty(p.shape, device=dev, dtype=p.dtype)
                 fresh.append((p, mg, g))
                 grads.append(g.data_ptr())
-        parts = max(nv.lib().mmt_rmsnorm_bwd_parts(T) * C, nv.lib().mmt_colsum_parts(T) * max(2 * inter, qw, C))
+        parts = 2 * nv.lib().mmt_rmsnorm_bwd_parts(T) * C + nv.lib().mmt_colsum_parts(T) * sum(
+            b.shape[0] for b in (P[2], P[4], P[7], P[9]) if b is not None)
         split = split_heads(T, s.n_q, s.n_kv)
         dx = torch.empty_like(x)
         scratch, addr = _carve([4 * T * inter, 2 * T * max(inter, qw), 2 * T * max(C, aw), 2 * T * C, 4 * s.n_q * T,
