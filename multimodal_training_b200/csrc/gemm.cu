@@ -1387,7 +1387,7 @@ void read_env_once() {
   }
   if (g_mt2_const < 0.0) {
     const char* e = getenv("MMT_GEMM_MT2_CONST");
-    g_mt2_const = e ? atof(e) : 4.06;
+    g_mt2_const = e ? atof(e) : 3.8;
   }
 }
 cudaEvent_t g_sk_event = nullptr;
@@ -1633,11 +1633,13 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
   // 256 (two accumulators that share every B tile: the main loop alternates between them, which keeps the tensor pipe
   // busier than back-to-back MMAs into one accumulator, but the two fill tensor memory and the epilogue is exposed);
   // width = 192 or 256 columns (narrower only for narrow outputs: a 128-wide MMA is bound by shared-memory reads).
-  // Cost of a candidate = waves x (k-blocks x c + e), in units of one 256 x 256 x 64 step, with c and e fitted (least
-  // squares over 200 sustained measurements on B200: the step's text shapes, the short-K vision shapes and the
-  // tensor-parallel shards, all layouts) per tile shape (rows x width: 128 x 256 c 0.568 e 0.86; 256 x 256 c 0.824
-  // e 4.06; 128 x 192 c 0.507 e 0.4; 256 x 192 c 0.726 e 2.61).  What it mostly decides is how well the tile count
-  // fills the 148 SMs.
+  // Cost of a candidate in us = waves x (k-blocks x c + e), with c and e from single GEMMs of 1600 to 16384 rows and K of
+  // 1280 to 6848 in a graph (rows x width: 128 x 256 c 0.39 e 0.5; 256 x 256 c 0.636 e 3.8; 128 x 192 c 0.33 e 0.6;
+  // 256 x 192 c 0.56 e 2.2).  c is close to what one SM's operand intake (about 110 GB/s) allows, so wide tiles win for
+  // long K; e is the exposed epilogue of a 256-row tile, so 128-row tiles win for short K.  A last wave that is partly
+  // empty has the L2 to itself and is up to a fifth faster.  What it mostly decides is how well the tile count fills
+  // the 148 SMs.  (Constants from the time when issuing paced the 128-row tiles preferred 256 rows more often: 16384 x
+  // 1280 x 1280 62.5 -> 50.6 us, 16384 x 1280 x 3840 135 -> 125, 6000 x 3840 x 1280 53.7 -> 49.1.)
   read_env_once();
   int mt = 1;
   const long kb = (K + BK - 1) / BK;
@@ -1645,13 +1647,13 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
   auto cost = [&](int m, int width) {
     const long tiles = (long)((M + 128 * m - 1) / (128 * m)) * ((N + width - 1) / width);
     const long full = tiles / sms, rem = tiles % sms;
-    double waves = (double)full + (rem ? 1.0 : 0.0);
-    if (rem && plain && width == 256 && sk_tiles_for((int)tiles, kb, sms, m) > 0)
-      waves = (double)full + (double)rem / sms + (m == 2 ? 16.0 : 8.0) / (double)kb;
     double c, e;
-    if (width == 256) { c = m == 2 ? 0.824 : 0.568; e = m == 2 ? g_mt2_const : 0.86; }
-    else              { c = m == 2 ? 0.726 : 0.507; e = m == 2 ? 2.61 : 0.4; }
-    return waves * ((double)kb * c + e);
+    if (width == 256) { c = m == 2 ? 0.636 : 0.39; e = m == 2 ? g_mt2_const : 0.5; }
+    else              { c = m == 2 ? 0.56 : 0.33; e = m == 2 ? 2.2 : 0.6; }
+    if (rem && plain && width == 256 && sk_tiles_for((int)tiles, kb, sms, m) > 0)
+      return ((double)full + (double)rem / sms + (m == 2 ? 16.0 : 8.0) / (double)kb) * ((double)kb * c + e);
+    const double last = rem ? kb * c * (0.8 + 0.2 * (double)rem / sms) + e : 0.0;
+    return full * ((double)kb * c + e) + last;
   };
   if (bn == 0 && g_force_bn) bn = g_force_bn;
   const bool choose = bn == 0 && g_force_mt == 0 && !g_use_pair;
