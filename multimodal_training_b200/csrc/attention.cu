@@ -102,28 +102,28 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
   const int pair = p.causal ? n_pairs - 1 - (int)blockIdx.x / p.n_q : (int)blockIdx.x % n_pairs;
   const int kv_head = head / (p.n_q / p.n_kv);
   const int xq = head * DIM, xk = (p.n_q + kv_head) * DIM, xv = (p.n_q + p.n_kv + kv_head) * DIM;
-  // blocks j in [first[w], last[w]) of 128 KV rows, counted from the first row that tile 0 sees, are visible to tile w
-  int q0[2], first[2], last[2];
-  int kv_base = 0;
+  // The CTA walks blocks of 128 KV rows; block j is worked on by tile w if first[w] <= j < last[w].  Tiles of one sequence
+  // start at the same row and share their blocks.  If the second tile starts in another sequence, its blocks follow those
+  // of the first one and are counted from its own first row: a tile's blocks, and with them its sums, do not depend on
+  // its neighbour.
+  int q0[2], first[2], last[2], lo_w[2] = {0, 0};
 #pragma unroll
   for (int w = 0; w < 2; ++w) {
     q0[w] = (pair * 2 + w) * BQ;
     first[w] = last[w] = 0;
     if (q0[w] < p.T) {
       const int q_last = min(q0[w] + BQ, p.T) - 1;
-      const int lo = p.seq_lo[q0[w]];
+      lo_w[w] = p.seq_lo[q0[w]];
       const int hi = p.causal ? min(p.seq_hi[q_last], q_last + 1) : p.seq_hi[q_last];
-      if (w == 0) kv_base = lo;
-      first[w] = (lo - kv_base) / BKV;
-      last[w] = (hi - kv_base + BKV - 1) / BKV;
+      if (w == 1 && lo_w[1] != lo_w[0]) first[1] = last[0];
+      last[w] = first[w] + (hi - lo_w[w] + BKV - 1) / BKV;
     }
-  }
-#pragma unroll
-  for (int w = 0; w < 2; ++w) {
     first[w] = warp_uniform(first[w]);
     last[w] = warp_uniform(last[w]);
+    lo_w[w] = warp_uniform(lo_w[w]);
   }
-  kv_base = warp_uniform(kv_base);
+  const int own1 = first[1] > 0 ? first[1] : 0x7fffffff;        // first block that is counted from tile 1's first row
+  auto block_row = [&](int j) { return j < own1 ? lo_w[0] + j * BKV : lo_w[1] + (j - own1) * BKV; };
   const int n_blocks = max(last[0], last[1]);
 
   if (warp == 8) {
@@ -140,7 +140,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
     for (int j = 0; j < n_blocks; ++j) {
       const int st = j & 1;
       const uint32_t free_parity = (uint32_t)(((j >> 1) & 1) ^ 1);
-      const int r0 = kv_base + j * BKV;
+      const int r0 = block_row(j);
       if (!mbar_wait_warp(&k_empty[st], free_parity, p.ew, 410)) break;
       load(sK + st * 2 * CHUNK, &k_full[st], xk, r0);
       if (j == 0 && last[1] > first[1]) load(sQ + 2 * CHUNK, &q_full[1], xq, q0[1]);
@@ -235,7 +235,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
       float m_ref = -INFINITY, l = 0.f;
       bool ok = true;
       for (int j = j0; j < j1; ++j) {
-        const int kv0 = kv_base + j * BKV;
+        const int kv0 = block_row(j);
         ok = __all_sync(0xffffffffu, mbar_wait(&s_full[w], (j - j0) & 1, p.ew, 610));
         if (!ok) break;
         tc_fence_after();
@@ -285,7 +285,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
         const float bias = (m_ref == -INFINITY) ? 0.f : -m_ref * sl2;
         const float2 bias2 = make_float2(bias, bias);
         // P = exp2(S * sl2 + bias) as bf16 pairs, written over the columns of S
-        float2 sum = make_float2(0.f, 0.f);
+        float sum = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           // the last 32 scores are read a second time instead of being held over the first 96: they and the packed
@@ -301,12 +301,12 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p, con
               if (!((vis[c] >> i) & 1u)) e.x = 0.f;
               if (!((vis[c] >> (i + 1)) & 1u)) e.y = 0.f;
             }
-            sum = add2(sum, e);
+            sum += e.x + e.y;
             pk[i >> 1] = pack_bf16x2(e.x, e.y);
           }
           tmem_st_32x32b_x16(s_addr + c * 16, pk);
         }
-        l += sum.x + sum.y;
+        l += sum;
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();

@@ -1,18 +1,19 @@
 // Attention over short sequences: packs of whole sequences of up to 128 rows together (the vision encoder's windows).
 //
-// The kernels of attention.cu and attention_bwd.cu walk KV blocks for a 128-row query tile.  When no sequence is longer
-// than a tile there is nothing to walk: with the rows cut at sequence boundaries instead of multiples of 128, one CTA
-// sees every query and every key of its rows.  So
+// The kernels of attention.cu and attention_bwd.cu walk KV blocks for a 128-row query tile.  When no sequence reaches out
+// of its tile there is nothing to walk: one CTA sees every query and every key of its rows.  So
 //   * forward needs one S and one PV product, 97 KB of shared memory and half of tensor memory: two CTAs per SM hide
-//     each other's load, softmax and store phases (the general kernel has one CTA per SM and, for rows that do not fall
-//     on multiples of 128, reads two or three KV blocks per tile);
+//     each other's load, softmax and store phases (the general kernel has one CTA per SM);
 //   * backward computes P and dS ONCE and takes all three gradients from them (five products where the dK/dV and dQ
 //     kernels need seven), reads Q, K, V and dO once, and forms delta = rowsum(out * dout) itself: one launch for three.
-// Measured in the kernels' own time, 64-row windows, 16384 patches, 16 heads of 80: forward 72.6 -> 50.2 us, backward
-// 276 -> 140 us; training step of five photos (9024 patches, windows cut at the edges) 77.9 -> 74.3 ms.
+// Measured in the kernels' own time, 64-row windows, 16384 patches, 16 heads of 80: forward 72.6 -> 50 us, backward
+// 276 -> 141 us; vision step of a 1792 x 1792 image 125.4 -> 121.7 ms.
 //
-// `items` holds (first row, rows) of every pack.  The rows of a pack beyond `rows` in its 128-row boxes belong to the
-// next packs; they are masked like any row of another sequence, and never written.
+// `items` holds (first row, rows) of every pack.  Packs are whole 128-row tiles (the last one may be shorter): batches in
+// which a sequence lies across a multiple of 128 rows go to the general kernels.  So every sum here runs over the same
+// keys in the same order as there, and a batch gives the same bits on both paths.  (Packs cut elsewhere were 5 % faster
+// for a step on photos, but a row's probabilities were then rounded relative to another maximum, and after 32 layers of
+// bf16 the gradients differed by as much as rounding noise does.)
 #include "attention_common.cuh"
 
 namespace {
@@ -138,7 +139,7 @@ attn_local_fwd_kernel(const __grid_constant__ CUtensorMap tm, const LocalParams 
       m = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       const float bias = m == -INFINITY ? 0.f : -m * sl2;
       const float2 bias2 = make_float2(bias, bias);
-      float2 sum = make_float2(0.f, 0.f);
+      float sum = 0.f;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t pk[16];
@@ -150,7 +151,7 @@ attn_local_fwd_kernel(const __grid_constant__ CUtensorMap tm, const LocalParams 
             float2 e = make_float2(exp2f(t.x), exp2f(t.y));
             if (!((vis[c] >> i) & 1u)) e.x = 0.f;
             if (!((vis[c] >> (i + 1)) & 1u)) e.y = 0.f;
-            sum = add2(sum, e);
+            sum += e.x + e.y;
             pk[i >> 1] = pack_bf16x2(e.x, e.y);
           }
         } else {
@@ -159,7 +160,7 @@ attn_local_fwd_kernel(const __grid_constant__ CUtensorMap tm, const LocalParams 
         }
         tmem_st_32x32b_x16(t_s + lane_addr + c * 16, pk);
       }
-      l = sum.x + sum.y;
+      l = sum;
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -309,23 +310,29 @@ attn_local_bwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
       lo -= r0;
       hi -= r0;
       lse_l2 = p.lse[(long)head * p.T + grow] * LOG2E;
-      // this thread's half of the row's delta
-      const long at = (long)grow * (p.n_q * DIM) + head * DIM + half * (DIM / 2);
-      uint4 o[DIM / 16], d[DIM / 16];
+      // delta = sum of out * dout in the order in which a warp with a pair of columns per lane adds it up (the lane's
+      // pairs, then lanes 16, 8, 4, 2 and 1 apart), so that it has the same bits as attn_delta_kernel's; this thread has
+      // the even or the odd lanes, and the last step joins the two
+      const long at = (long)grow * (p.n_q * DIM) + head * DIM;
+      float lane_sum[16];
 #pragma unroll
-      for (int i = 0; i < DIM / 16; ++i) {
-        o[i] = *reinterpret_cast<const uint4*>(p.out + at + i * 8);
-        d[i] = *reinterpret_cast<const uint4*>(p.dout + at + i * 8);
-      }
+      for (int i = 0; i < 16; ++i) lane_sum[i] = 0.f;
 #pragma unroll
-      for (int i = 0; i < DIM / 16; ++i) {
-        const uint32_t ow[4] = {o[i].x, o[i].y, o[i].z, o[i].w}, dw[4] = {d[i].x, d[i].y, d[i].z, d[i].w};
+      for (int i = 0; i < DIM / 8; ++i) {
+        const uint4 o = *reinterpret_cast<const uint4*>(p.out + at + i * 8);
+        const uint4 d = *reinterpret_cast<const uint4*>(p.dout + at + i * 8);
+        const uint32_t ow[2] = {half ? o.y : o.x, half ? o.w : o.z}, dw[2] = {half ? d.y : d.x, half ? d.w : d.z};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 2; ++j) {
           const float2 a = unpack_bf16x2(ow[j]), b = unpack_bf16x2(dw[j]);
-          part += a.x * b.x + a.y * b.y;
+          lane_sum[(2 * i + j) & 15] += a.x * b.x + a.y * b.y;
         }
       }
+#pragma unroll
+      for (int step = 8; step > 0; step >>= 1)
+#pragma unroll
+        for (int i = 0; i < step; ++i) lane_sum[i] += lane_sum[i + step];
+      part = lane_sum[0];
     }
     sDelta[half * 128 + row] = part;
     quadrant_bar_sync<2>(q4);

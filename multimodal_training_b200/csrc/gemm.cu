@@ -1437,10 +1437,12 @@ struct SmallTile {
 //   128 x 256         0.360   1.2   |             0.326   6.3   |             0.350   4.4
 //   256 x 192         0.515   3.4   |
 //   256 x 256         0.600   5.3   |
-// Measured (us, wave model -> this): 256 x 1280 x 3424 23.3 -> 9.1, 256 x 3840 x 1280 12.0 -> 8.7, 256 x 6848 x 1280
-// 12.5 -> 10.3, 443 x 2048 x 11008 62.0 -> 23.6, weight gradient 1280 x 1280 x 4096 25.8 -> 17.6.
+// Measured (us, wave model -> this): 256 x 1280 x 3424 23.3 -> 16.5, 256 x 3840 x 1280 12.0 -> 9.2, 256 x 6848 x 1280
+// 12.5 -> 10.3, 1024 x 1280 x 3424 23.8 -> 18.5, weight gradient 1280 x 1280 x 4096 25.8 -> 17.6.
 // `mt`, `bn` is the choice of the wave model, which stays when nothing is cheaper.
-SmallTile small_tile(int M, int N, long kb, int sms, int mt, int bn) {
+SmallTile small_tile(int M, int N, long kb, int sms, int mt, int bn, bool may_split) {
+  // Only weight gradients are split: their values are final.  A split activation or input gradient is as accurate, but its
+  // sums are rounded in another order, and the bf16 layers behind it carry the difference through the whole model.
   static const double c1[4] = {0.235, 0.245, 0.335, 0.360}, e1[4] = {0.0, 0.2, 0.0, 1.2};
   static const double c2[4] = {0.190, 0.190, 0.262, 0.326}, e2[4] = {0.0, 1.2, 3.6, 6.3};
   static const double c4[4] = {0.230, 0.225, 0.285, 0.350}, e4[4] = {0.1, 2.1, 3.1, 4.4};
@@ -1458,6 +1460,7 @@ SmallTile small_tile(int M, int N, long kb, int sms, int mt, int bn) {
       best = {1, width, 1};
       t_best = kb * c1[i] + e1[i];
     }
+    if (!may_split) continue;
     if (tiles <= slots2 && kb >= 4 && (kb + 1) / 2 * c2[i] + e2[i] < t_best) {
       best = {1, width, 2};
       t_best = (kb + 1) / 2 * c2[i] + e2[i];
@@ -1685,7 +1688,7 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
     // The model above weighs full waves.  A grid that does not fill one is decided by its longest chain of k-blocks.
     const long tiles = (long)((M + 128 * mt - 1) / (128 * mt)) * ((N + bn - 1) / bn);
     if (tiles <= sms) {
-      const SmallTile t = small_tile(M, N, kb, sms, mt, bn);
+      const SmallTile t = small_tile(M, N, kb, sms, mt, bn, a_mn && b_mn);
       mt = t.mt; bn = t.bn; split = t.split;
     }
   }

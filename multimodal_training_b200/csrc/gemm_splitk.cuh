@@ -1,13 +1,13 @@
 // Split-K GEMM for grids that leave most SMs idle; included by gemm.cu (same parameters, operand layouts and ring).
 //
-// A small output (256 rows of activations, a weight gradient of a square projection) has 10 to 70 tiles for 148 SMs, and
+// The gradient of a square projection has 25 to 70 tiles for 148 SMs, and
 // one SM takes operands in at about 100 GB/s whatever the tile: the GEMM's time is then its longest K loop.  Here a
 // cluster of S CTAs shares one 128 x BN tile: CTA r multiplies the r-th part of K, then every CTA owns BN / S of the
 // tile's columns, receives the other CTAs' fp32 partial sums of those columns in its (by then idle) operand ring through
 // distributed shared memory, adds them in rank order and finishes the columns.  The reduction is spread over all S CTAs,
 // needs no workspace, no flags and no second launch, and its result does not depend on timing.
-// Measured: 256 x 1280 x 3424 (14 tiles of 192 columns unsplit) 23.3 -> 9.1 us as 40 tiles of 64 columns over 2 CTAs;
-// the exchange costs 1 to 6 us, growing with the tile, so wide tiles are split for long K only (small_tile in gemm.cu).
+// Measured: weight gradient 1280 x 1280 x 4096 25.8 (unsplit) -> 17.6 us as 70 tiles of 192 columns over 2 CTAs; the
+// exchange costs 1 to 6 us, growing with the tile, so wide tiles are split for long K only (small_tile in gemm.cu).
 
 MMT_DEVICE void st_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d)

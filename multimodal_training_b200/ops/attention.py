@@ -17,7 +17,7 @@ import torch
 from . import native as nv
 
 BACKEND = "sm100"
-LOCAL_ROWS = 128      # rows of one tile: batches of sequences up to this length take csrc/attention_local.cu
+LOCAL_ROWS = 128      # rows of a tile: batches whose sequences stay inside tiles take csrc/attention_local.cu
 
 
 def set_backend(name: str) -> None:
@@ -37,6 +37,7 @@ class SeqInfo:
     _lo: torch.Tensor | None = None
     _hi: torch.Tensor | None = None
     _packs: torch.Tensor | None = None
+    _in_tiles: bool | None = None
 
     @classmethod
     def from_list(cls, cu: list[int], device) -> "SeqInfo":
@@ -69,25 +70,15 @@ class SeqInfo:
 
 
     def packs(self) -> torch.Tensor | None:
-        """(first row, rows) of consecutive whole sequences taken together up to LOCAL_ROWS rows (int32, device), or
-        None when a sequence is longer than that: what the kernels for short sequences work on."""
-        if self._packs is None and 0 < self.max_len <= LOCAL_ROWS:
-            self._packs = torch.tensor(pack_sequences(self.host, LOCAL_ROWS), dtype=torch.int32).to(
-                self.device, non_blocking=True)
+        """(first row, rows) of the 128-row tiles (int32, device), or None when a sequence reaches out of its tile:
+        what the kernels for short sequences work on."""
+        if self._packs is None and self.total > 0 and self._in_tiles is None:
+            self._in_tiles = all(a == b or a // LOCAL_ROWS == (b - 1) // LOCAL_ROWS
+                                 for a, b in zip(self.host[:-1], self.host[1:]))
+        if self._packs is None and self._in_tiles:
+            tiles = [(r, min(LOCAL_ROWS, self.total - r)) for r in range(0, self.total, LOCAL_ROWS)]
+            self._packs = torch.tensor(tiles, dtype=torch.int32).to(self.device, non_blocking=True)
         return self._packs
-
-
-def pack_sequences(cu: list[int], limit: int) -> list[tuple[int, int]]:
-    """Cuts the rows of ``cu`` at sequence boundaries into pieces of at most ``limit`` rows (no sequence is longer)."""
-    out = []
-    first = cu[0]
-    for a, b in zip(cu[:-1], cu[1:]):
-        if b - first > limit:
-            out.append((first, a - first))
-            first = a
-    if cu[-1] > first:
-        out.append((first, cu[-1] - first))
-    return out
 
 
 class _LibAttentionFn(torch.autograd.Function):

@@ -42,9 +42,33 @@ def test_growing_scores_rescale():
     assert ((out.float() - ref).abs().max() / ref.abs().max()).item() < TOL
 
 
-def test_packs_cover_all_rows_once():
-    from multimodal_training_b200.ops.attention import pack_sequences
-    for cu in ([0, 64, 128, 192], [0, 1, 2, 130], [0, 128, 256], [0, 100, 100, 200, 230], [0, 7]):
-        packs = pack_sequences(cu, 128)
-        assert [r for a, n in packs for r in range(a, a + n)] == list(range(cu[-1]))
-        assert all(0 < n <= 128 and a in cu and a + n in cu for a, n in packs)
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,causal", [(80, False), (128, True)])
+def test_short_sequences_have_the_bits_of_the_general_kernels(dim, causal, monkeypatch):
+    from multimodal_training_b200.ops import functional as F
+    from multimodal_training_b200.ops.attention import SeqInfo
+    cu = [0, 64, 128, 140, 256, 256, 300, 383, 384, 400]
+    torch.manual_seed(5)
+    x = torch.randn(cu[-1], 9 * dim, device="cuda").bfloat16()
+    dout = torch.randn(cu[-1], 3 * dim, device="cuda").bfloat16()
+
+    def both():
+        q = x.clone().requires_grad_()
+        out = F.attention(q, 3, 3, dim, SeqInfo.from_list(cu, "cuda"), causal=causal)
+        out.backward(dout)
+        return out.detach(), q.grad
+
+    local = both()
+    monkeypatch.setattr(SeqInfo, "packs", lambda self: None)
+    general = both()
+    assert torch.equal(local[0], general[0]) and torch.equal(local[1], general[1])
+
+
+def test_which_batches_stay_inside_tiles():
+    from multimodal_training_b200.ops.attention import SeqInfo
+    for cu, inside in (([0, 64, 128, 192], True), ([0, 128, 256, 300], True), ([0, 100, 128, 128, 130], True), ([0, 7], True),
+                       ([0, 129], False), ([0, 100, 140], False), ([0, 64, 128, 160, 288], False), ([0], False)):
+        packs = SeqInfo.from_list(cu, "cpu").packs()
+        assert (packs is not None) == inside
+        if inside:
+            assert [r for a, n in packs.tolist() for r in range(a, a + n)] == list(range(cu[-1]))
