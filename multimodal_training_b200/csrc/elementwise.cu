@@ -562,6 +562,14 @@ __global__ void __launch_bounds__(kCeThreads) ce_stats_kernel(const bf16* __rest
   const long row = blockIdx.x;
   const bf16* l = logits + row * ld;
   const int nvec = V >> 3;
+  if (labels[row] < 0) {            // an ignored row takes no part in the loss; its statistics only have to be finite
+    if (threadIdx.x == 0) {
+      omax[row] = 0.f;
+      osum[row] = 1.f;
+      otgt[row] = 0.f;
+    }
+    return;
+  }
   float m = -INFINITY, s = 0.f;
   for (int c = threadIdx.x; c < nvec; c += kCeThreads) {
     float v[8];
@@ -591,17 +599,27 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* __restrict__ 
                                                             const float* __restrict__ gmax,
                                                             const float* __restrict__ gsum,
                                                             const float* __restrict__ scale_ptr, int V, long ld,
-                                                            long vocab_lo) {
+                                                            long vocab_lo, const int* __restrict__ cnt, int base) {
   grid_dependency_sync();
   const long row = blockIdx.x;
   bf16* l = logits + row * ld;
   const int nvec = V >> 3;
+  if (cnt) {
+    // compacted rows: those behind the last valid one are not read again, except that the weight gradient's last block
+    // of 64 rows (the first one if there is no valid row) has to end in zeros
+    const int n = max(*cnt - base, 0);
+    if (row >= n && row >= max((n + 63) / 64 * 64, 64)) return;
+  }
   const long lab_g = labels[row];
-  const bool valid = lab_g >= 0;
+  if (lab_g < 0) {
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (int c = threadIdx.x; c < nvec; c += kCeThreads) *reinterpret_cast<uint4*>(l + c * 8) = zero;
+    return;
+  }
   const long lab = lab_g - vocab_lo;
-  const float scale = valid ? *scale_ptr : 0.f;
+  const float scale = *scale_ptr;
   const float m = gmax[row];
-  const float inv = valid ? 1.f / gsum[row] : 0.f;
+  const float inv = 1.f / gsum[row];
   for (int c = threadIdx.x; c < nvec; c += kCeThreads) {
     float v[8];
     load8(l + c * 8, v);
@@ -613,6 +631,44 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* __restrict__ 
     }
     store8(l + c * 8, v);
   }
+}
+
+// ----------------------------------------------------------------------------
+// Rows with a label, in order: src[j] = the j-th such row and its label, -1 and -1 behind the last; pos[t] = j or -1;
+// *count = their number.  One CTA: a few thousand labels are a few microseconds, and nothing waits for the host.
+// ----------------------------------------------------------------------------
+constexpr int kCompactThreads = 1024;
+__global__ void __launch_bounds__(kCompactThreads) compact_labels_kernel(const long* __restrict__ labels, long n,
+                                                                        long* __restrict__ src, long* __restrict__ lab,
+                                                                        long* __restrict__ pos, int* __restrict__ count) {
+  grid_dependency_sync();
+  __shared__ int warp_total[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int base = 0;
+  for (long t0 = 0; t0 < n; t0 += kCompactThreads) {
+    const long t = t0 + threadIdx.x;
+    const long l = t < n ? labels[t] : -1;
+    const unsigned ballot = __ballot_sync(0xffffffffu, l >= 0);
+    if (lane == 0) warp_total[warp] = __popc(ballot);
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) {
+      const int v = warp_total[w];
+      before += w < warp ? v : 0;
+      total += v;
+    }
+    const int j = base + before + __popc(ballot & ((1u << lane) - 1u));
+    if (t < n) pos[t] = l >= 0 ? j : -1;
+    if (l >= 0) {
+      src[j] = t;
+      lab[j] = l;
+    }
+    base += total;
+    __syncthreads();
+  }
+  for (long j = base + threadIdx.x; j < n; j += kCompactThreads) src[j] = lab[j] = -1;
+  if (threadIdx.x == 0) *count = base;
 }
 
 // ----------------------------------------------------------------------------
@@ -933,14 +989,20 @@ int mmt_ce_stats(const void* logits, const long* labels, float* omax, float* osu
                                                                 vocab_lo);
   return (int)cudaGetLastError();
 }
+// cnt (optional): rows [0, *cnt - base) are valid, the rest is not needed (see ce_grad_kernel).
 int mmt_ce_grad(void* logits, const long* labels, const float* gmax, const float* gsum, const float* scale_ptr,
-                long rows, int V, long ld, long vocab_lo, void* stream) {
+                long rows, int V, long ld, long vocab_lo, const int* cnt, int base, void* stream) {
   if (V % 8 || ld % 8) return -2;
   if (rows == 0) return 0;
   launch_dependent(ce_grad_kernel, (unsigned)rows, kCeThreads, 0, ST(stream),
                      BF(logits), labels, gmax, gsum, scale_ptr, V, ld,
-                                                               vocab_lo);
+                                                               vocab_lo, cnt, base);
   return (int)cudaGetLastError();
+}
+
+int mmt_compact_labels(const long* labels, long n, long* src, long* lab, long* pos, int* count, void* stream) {
+  if (n < 0 || n > 0x7fffffffL) return -5;
+  return (int)launch_dependent(compact_labels_kernel, 1, kCompactThreads, 0, ST(stream), labels, n, src, lab, pos, count);
 }
 
 int mmt_adamw(void* p, const void* g, float* master, float* m, float* v, long n, long n_decay, float lr, float b1,

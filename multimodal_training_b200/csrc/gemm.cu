@@ -67,6 +67,13 @@ struct GemmParams {
   int group_m, tiles_n;           // raster: m-tiles per band (0 = all), number of n-tiles
   uint32_t mn_lbo, mn_sbo, mn_kstep;  // descriptor constants of MN-major tiles
   MmtErrorWord* ew;
+  // --- number of rows (cnt_k == 0) or length of K (cnt_k == 1) known on the device only: min(max(*cnt - cnt_base, 0), M or K).
+  //     Rows: tiles beyond the last row are not computed, and the launch does nothing unless the count falls into one of
+  //     its buckets (bit (rows - 1) / cnt_bucket of cnt_mask).  K: k-blocks beyond the count are not read; the rest of the
+  //     last one has to hold zeros (also the first one when the count is 0).  nullptr: M and K are what they are.
+  const int* cnt;
+  int cnt_base, cnt_k, cnt_bucket;
+  uint32_t cnt_mask;
   int local_only;                 // no waits on other CTAs or peers: this launch may overlap its neighbours' ends
   // --- stream-K for the last partial wave: the final `sk_tiles` tiles are cut along K into gridDim.x equal runs of
   //     k-blocks, one per CTA; a CTA that does not reach the end of a tile leaves its fp32 partial in `sk_ws`
@@ -744,10 +751,6 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     clk_c0 = clock64();
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(clk_t0));
   }
-  const int tiles_m = (p.M + BMT - 1) / BMT;
-  const int tiles_n = (p.N + BN - 1) / BN;
-  const int ntiles = tiles_m * tiles_n;
-  const int KB = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
@@ -773,6 +776,16 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   grid_dependency_wait();
+  int m_rows = p.M, k_len = p.K;
+  if (p.cnt) {
+    const int n = warp_uniform(min(max(*p.cnt - p.cnt_base, 0), p.cnt_k ? p.K : p.M));
+    if (p.cnt_k) k_len = max(n, 1);
+    else m_rows = n > 0 && ((p.cnt_mask >> ((n - 1) / p.cnt_bucket)) & 1u) ? n : 0;
+  }
+  const int tiles_m = (m_rows + BMT - 1) / BMT;
+  const int tiles_n = (p.N + BN - 1) / BN;
+  const int ntiles = tiles_m * tiles_n;
+  const int KB = (k_len + BK - 1) / BK;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -1618,9 +1631,30 @@ extern "C" void mmt_gemm_set_comm(const MmtGemmComm* c) { g_comm = c; }
 //   act         : 0 none, 1 GELU
 //   bn          : 0 = choose, else one of 64/128/192/256
 // Returns 0 or a CUDA / driver error code (negative: argument error).
-extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* bias, const void* residual, int M,
-                             int N, int K, int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int act,
-                             int accumulate, int out_f32, float alpha, int bn, void* stream) {
+// A count that only the device knows (GemmParams::cnt) and, for a count of rows, the tile of this launch.
+struct GemmCount {
+  const int* cnt;
+  int base, is_k, bucket;
+  uint32_t mask;
+  int mt, bn;
+};
+
+// Model of the persistent kernel's time, see gemm_call.
+static double wave_cost(int M, int N, long kb, int sms, int m, int width, bool stream_k) {
+  const long tiles = (long)((M + 128 * m - 1) / (128 * m)) * ((N + width - 1) / width);
+  const long full = tiles / sms, rem = tiles % sms;
+  double c, e;
+  if (width == 256) { c = m == 2 ? 0.636 : 0.39; e = m == 2 ? g_mt2_const : 0.5; }
+  else              { c = m == 2 ? 0.56 : 0.33; e = m == 2 ? 2.2 : 0.6; }
+  if (rem && stream_k && width == 256 && sk_tiles_for((int)tiles, kb, sms, m) > 0)
+    return ((double)full + (double)rem / sms + (m == 2 ? 16.0 : 8.0) / (double)kb) * ((double)kb * c + e);
+  const double last = rem ? kb * c * (0.8 + 0.2 * (double)rem / sms) + e : 0.0;
+  return full * ((double)kb * c + e) + last;
+}
+
+static int gemm_call(const void* A, const void* B, void* C, const void* bias, const void* residual, int M, int N, int K,
+                     int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int act, int accumulate, int out_f32,
+                     float alpha, int bn, const GemmCount* count, void* stream) {
   // collective roles belong to THIS call only: take them before any early return, so that a call that fails its
   // argument checks cannot leave them behind for an unrelated GEMM
   const MmtGemmComm* comm = g_comm;
@@ -1647,19 +1681,9 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
   int mt = 1;
   const long kb = (K + BK - 1) / BK;
   const bool plain = comm == nullptr;
-  auto cost = [&](int m, int width) {
-    const long tiles = (long)((M + 128 * m - 1) / (128 * m)) * ((N + width - 1) / width);
-    const long full = tiles / sms, rem = tiles % sms;
-    double c, e;
-    if (width == 256) { c = m == 2 ? 0.636 : 0.39; e = m == 2 ? g_mt2_const : 0.5; }
-    else              { c = m == 2 ? 0.56 : 0.33; e = m == 2 ? 2.2 : 0.6; }
-    if (rem && plain && width == 256 && sk_tiles_for((int)tiles, kb, sms, m) > 0)
-      return ((double)full + (double)rem / sms + (m == 2 ? 16.0 : 8.0) / (double)kb) * ((double)kb * c + e);
-    const double last = rem ? kb * c * (0.8 + 0.2 * (double)rem / sms) + e : 0.0;
-    return full * ((double)kb * c + e) + last;
-  };
+  auto cost = [&](int m, int width) { return wave_cost(M, N, kb, sms, m, width, plain); };
   if (bn == 0 && g_force_bn) bn = g_force_bn;
-  const bool choose = bn == 0 && g_force_mt == 0 && !g_use_pair;
+  const bool choose = bn == 0 && g_force_mt == 0 && !g_use_pair && !count;
   if (bn == 0 && N <= 192) bn = N > 128 ? 192 : (N > 64 ? 128 : 64);
   if (bn == 0) {
     double best = 1e30;
@@ -1680,8 +1704,13 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
   }
   if (bn == 256 && M >= 256 && (g_force_mt == 3 || (g_use_pair && g_force_mt == 0)) && !(comm && (comm->fwd_peers > 0 || comm->sc_row || comm->kf_flags)))
     mt = 3;   // 2-CTA kernel
+  if (count && count->mt) {
+    mt = count->mt;
+    bn = count->bn;
+  }
+  if (count && mt == 3) mt = 2;                          // the pair kernel does not look at counts
   int split = 1;
-  if (plain && mt != 3 && g_force_split > 1) {
+  if (plain && !count && mt != 3 && g_force_split > 1) {
     split = g_force_split;
     mt = 1;
   } else if (plain && choose && !g_sk_mode && g_force_split < 0) {
@@ -1713,6 +1742,11 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
   p.a_mn = a_mn; p.b_mn = b_mn;
   p.mn_lbo = g_mn_lbo; p.mn_sbo = g_mn_sbo; p.mn_kstep = g_mn_kstep;
   p.ew = mmt_error_word();
+  p.cnt = count ? count->cnt : nullptr;
+  p.cnt_base = count ? count->base : 0;
+  p.cnt_k = count ? count->is_k : 0;
+  p.cnt_bucket = count ? count->bucket : 1;
+  p.cnt_mask = count ? count->mask : 0;
   p.clk = g_clk;
   p.dbg = g_dbg;  // read through MMT_DBG only
   p.tiles_n = (N + bn - 1) / bn;
@@ -1783,7 +1817,7 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
   p.sk_flags = nullptr;
   p.sk_epoch = 0;
   bool sk_on = false;
-  if (!comm && mt != 3 && split == 1 && !(MMT_DBG & 1)) {
+  if (!comm && !count && mt != 3 && split == 1 && !(MMT_DBG & 1)) {
     const int tiles = ((M + bmt - 1) / bmt) * ((N + bn - 1) / bn);
     const int skt = sk_tiles_for(tiles, (K + BK - 1) / BK, sms, mt);
     if (skt > 0 && sk_ready()) {
@@ -1869,6 +1903,49 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
     g_sk_stream = st;
   }
   return rc;
+}
+
+extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* bias, const void* residual, int M,
+                             int N, int K, int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int act,
+                             int accumulate, int out_f32, float alpha, int bn, void* stream) {
+  return gemm_call(A, B, C, bias, residual, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, act, accumulate, out_f32, alpha, bn,
+                   nullptr, stream);
+}
+
+// The same product over the first min(max(*cnt - base, 0), M) rows of A and C (is_k == 0; later rows of C are undefined)
+// or over that many of the K rows of MN-major A and B (is_k == 1; see GemmParams::cnt for the zeros it needs).  The host
+// does not know the count, and which tile is best depends on it: a row count is cut into up to 32 buckets, and every
+// tile that is the best of some bucket is launched; the launches that the count does not belong to return at once.
+extern "C" int mmt_gemm_bf16_counted(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                                     int a_mn, int b_mn, int accumulate, const int* cnt, int base, int is_k,
+                                     void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  GemmCount c = {cnt, base, is_k, 1, 0u, 0, 0};
+  if (is_k)
+    return gemm_call(A, B, C, nullptr, nullptr, M, N, K, lda, ldb, ldc, 0, a_mn, b_mn, 0, accumulate, 0, 1.f, 0, &c, stream);
+  read_env_once();
+  const int sms = mmt_sm_count();
+  const long kb = (K + BK - 1) / BK;
+  c.bucket = ((M + 31) / 32 + 127) / 128 * 128;
+  uint32_t mask[4] = {0, 0, 0, 0};                       // 128 x 192, 128 x 256, 256 x 192, 256 x 256
+  for (int b = 0; b * c.bucket < M; ++b) {
+    int best = 0;
+    for (int t = 1; t < 4; ++t)
+      if (wave_cost(min((b + 1) * c.bucket, M), N, kb, sms, 1 + t / 2, 192 + 64 * (t & 1), false) <
+          wave_cost(min((b + 1) * c.bucket, M), N, kb, sms, 1 + best / 2, 192 + 64 * (best & 1), false))
+        best = t;
+    mask[best] |= 1u << b;
+  }
+  for (int t = 0; t < 4; ++t) {
+    if (!mask[t]) continue;
+    c.mask = mask[t];
+    c.mt = 1 + t / 2;
+    c.bn = 192 + 64 * (t & 1);
+    const int rc = gemm_call(A, B, C, nullptr, nullptr, M, N, K, lda, ldb, ldc, 0, a_mn, b_mn, 0, accumulate, 0, 1.f, c.bn,
+                             &c, stream);
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 // Tuning knob: 1 = stream-K for partial last waves, 0 = whole tiles only (default).
