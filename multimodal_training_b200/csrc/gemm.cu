@@ -1103,7 +1103,7 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   }
 }
 
-#include "gemm_splitk.cuh"
+#include "gemm_small.cuh"
 
 // ------------------------------------------------------------------------------------
 // 2-CTA kernel (cta_group::2): a pair of CTAs on neighbouring SMs computes one 256 x 256 tile.
@@ -1430,57 +1430,49 @@ int sk_tiles_for(int tiles, long kb, int sms, int mt) {
 
 int g_force_bn = 0;   // 0 = choose, else the tile width (64 / 128 / 192 / 256) of every following GEMM
 int g_force_mt = 0;   // 0 = choose, 1 / 2 = force the number of 128-row accumulators per tile, 3 = 2-CTA kernel
-int g_force_split = -1;   // -1 = choose, 1 = never split K, 2 / 4 = split every plain GEMM over that many CTAs
+int g_force_small = -1;   // -1 = choose, 0 = persistent kernel only, 1 = one tile per CTA
 int g_use_pair = 0;
 int g_group_m = 0;
 unsigned long long* g_clk = nullptr;
 int g_dbg = 0;
 
 struct SmallTile {
-  int mt, bn, split;
+  int mt, bn;
+  bool small;             // one tile per CTA (gemm_small.cuh) instead of the persistent kernel
 };
 
-// Tile shape and split of K for a grid of at most one wave: microseconds = k-blocks of a CTA x c + e, fitted to single
-// GEMMs in a graph (256 to 4096 rows, K 512 to 11008, all layouts) -- e holds what grows with the tile: the exposed
-// epilogue of a 256-row tile, the exchange of a split one.
-//   rows x width        c      e    | over 2 CTAs   c      e    | over 4 CTAs   c      e
-//   128 x  64         0.235   0.0   |             0.190   0.0   |             0.230   0.1
-//   128 x 128         0.245   0.2   |             0.190   1.2   |             0.225   2.1
-//   128 x 192         0.335   0.0   |             0.262   3.6   |             0.285   3.1
-//   128 x 256         0.360   1.2   |             0.326   6.3   |             0.350   4.4
-//   256 x 192         0.515   3.4   |
-//   256 x 256         0.600   5.3   |
-// Measured (us, wave model -> this): 256 x 1280 x 3424 23.3 -> 16.5, 256 x 3840 x 1280 12.0 -> 9.2, 256 x 6848 x 1280
-// 12.5 -> 10.3, 1024 x 1280 x 3424 23.8 -> 18.5, weight gradient 1280 x 1280 x 4096 25.8 -> 17.6.
+// Tile shape for a grid of at most one wave: microseconds = k-blocks x c + e, fitted to single GEMMs in a graph (144 to
+// 4096 rows, K 512 to 11008, all layouts) -- e holds what grows with the tile, such as the exposed epilogue of 256 rows.
+//   rows x width   persistent c  e | one tile a CTA c  e
+//   128 x  64        0.235   0.0   |   0.177  -1.0
+//   128 x 128        0.245   0.2   |   0.190   0.8
+//   128 x 192        0.335   0.0   |   0.255   1.6
+//   128 x 256        0.360   1.2   |   0.330   6.3
+//   256 x 192        0.515   3.4   |
+//   256 x 256        0.600   5.3   |
+// (One tile a CTA: no tiles to step through, which a narrow tile notices; an epilogue that nothing runs beside and that
+// stores 32-byte pieces, which a wide tile notices.)
+// Measured (us, wave model -> this): 256 x 1280 x 3424 23.3 -> 12.6, 256 x 3840 x 1280 12.0 -> 7.4, 256 x 6848 x 1280
+// 12.5 -> 10.3, 443 x 2048 x 11008 62.0 -> 33.2.  Sharing K between CTAs would give 9.1, 8.7, 10.3 and 23.6, and 17.6
+// instead of 21.3 for the weight gradient 1280 x 1280 x 4096, but the sums would be added in another order: as accurate,
+// and yet the bf16 layers (or optimizer steps) behind them turn any difference into one as large as rounding noise.
 // `mt`, `bn` is the choice of the wave model, which stays when nothing is cheaper.
-SmallTile small_tile(int M, int N, long kb, int sms, int mt, int bn, bool may_split) {
-  // Only weight gradients are split: their values are final.  A split activation or input gradient is as accurate, but its
-  // sums are rounded in another order, and the bf16 layers behind it carry the difference through the whole model.
+SmallTile small_tile(int M, int N, long kb, int sms, int mt, int bn) {
+  static const double c0[4] = {0.177, 0.190, 0.255, 0.330}, e0[4] = {-1.0, 0.8, 1.6, 6.3};
   static const double c1[4] = {0.235, 0.245, 0.335, 0.360}, e1[4] = {0.0, 0.2, 0.0, 1.2};
-  static const double c2[4] = {0.190, 0.190, 0.262, 0.326}, e2[4] = {0.0, 1.2, 3.6, 6.3};
-  static const double c4[4] = {0.230, 0.225, 0.285, 0.350}, e4[4] = {0.1, 2.1, 3.1, 4.4};
-  SmallTile best = {mt, bn, 1};
+  SmallTile best = {mt, bn, false};
   double t_best = mt == 2 ? (bn == 256 ? kb * 0.600 + 5.3 : kb * 0.515 + 3.4) : kb * c1[bn / 64 - 1] + e1[bn / 64 - 1];
   for (int i = 0; i < 4; ++i) {
     const int width = 64 * (i + 1);
     if (i > 0 && width - 64 >= N) break;                       // the narrower tile already holds every column
-    const long tiles = (long)((M + 127) / 128) * ((N + width - 1) / width);
-    const int slots2 = i == 0 ? split_slots<64, 2>() : (i == 1 ? split_slots<128, 2>()
-                                                        : (i == 2 ? split_slots<192, 2>() : split_slots<256, 2>()));
-    const int slots4 = i == 0 ? split_slots<64, 4>() : (i == 1 ? split_slots<128, 4>()
-                                                        : (i == 2 ? split_slots<192, 4>() : split_slots<256, 4>()));
-    if (tiles <= sms && kb * c1[i] + e1[i] < t_best) {
-      best = {1, width, 1};
+    if ((long)((M + 127) / 128) * ((N + width - 1) / width) > sms) continue;
+    if (kb * c1[i] + e1[i] < t_best) {
+      best = {1, width, false};
       t_best = kb * c1[i] + e1[i];
     }
-    if (!may_split) continue;
-    if (tiles <= slots2 && kb >= 4 && (kb + 1) / 2 * c2[i] + e2[i] < t_best) {
-      best = {1, width, 2};
-      t_best = (kb + 1) / 2 * c2[i] + e2[i];
-    }
-    if (tiles <= slots4 && kb >= 8 && (kb + 3) / 4 * c4[i] + e4[i] < t_best) {
-      best = {1, width, 4};
-      t_best = (kb + 3) / 4 * c4[i] + e4[i];
+    if (kb * c0[i] + e0[i] < t_best) {
+      best = {1, width, true};
+      t_best = kb * c0[i] + e0[i];
     }
   }
   return best;
@@ -1546,7 +1538,7 @@ int cached_tmap_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t o
 // Tuning knob: 0 = choose per call, 1 = 128-row tiles, 2 = 256-row tiles in one CTA, 3 = 2-CTA kernel.
 extern "C" void mmt_gemm_force_mt(int mt) { g_force_mt = mt; }
 
-extern "C" void mmt_gemm_force_split(int s) { g_force_split = s; }
+extern "C" void mmt_gemm_force_small(int on) { g_force_small = on; }
 // Tuning knob: tile width of every following GEMM (0 = choose per call).
 extern "C" void mmt_gemm_force_bn(int bn) { g_force_bn = bn; }
 // Raster band height in m-tiles (0 = choose, -1 = one band: m-fastest over the whole matrix).
@@ -1709,16 +1701,16 @@ static int gemm_call(const void* A, const void* B, void* C, const void* bias, co
     bn = count->bn;
   }
   if (count && mt == 3) mt = 2;                          // the pair kernel does not look at counts
-  int split = 1;
-  if (plain && !count && mt != 3 && g_force_split > 1) {
-    split = g_force_split;
+  bool small = false;
+  if (plain && !count && mt != 3 && g_force_small == 1) {
+    small = true;
     mt = 1;
-  } else if (plain && choose && !g_sk_mode && g_force_split < 0) {
+  } else if (plain && choose && !g_sk_mode && g_force_small < 0) {
     // The model above weighs full waves.  A grid that does not fill one is decided by its longest chain of k-blocks.
     const long tiles = (long)((M + 128 * mt - 1) / (128 * mt)) * ((N + bn - 1) / bn);
     if (tiles <= sms) {
-      const SmallTile t = small_tile(M, N, kb, sms, mt, bn, a_mn && b_mn);
-      mt = t.mt; bn = t.bn; split = t.split;
+      const SmallTile t = small_tile(M, N, kb, sms, mt, bn);
+      mt = t.mt; bn = t.bn; small = t.small;
     }
   }
   const int bmt = mt == 3 ? BM : BM * mt;              // rows per TMA box of A
@@ -1817,7 +1809,7 @@ static int gemm_call(const void* A, const void* B, void* C, const void* bias, co
   p.sk_flags = nullptr;
   p.sk_epoch = 0;
   bool sk_on = false;
-  if (!comm && !count && mt != 3 && split == 1 && !(MMT_DBG & 1)) {
+  if (!comm && !count && mt != 3 && !small && !(MMT_DBG & 1)) {
     const int tiles = ((M + bmt - 1) / bmt) * ((N + bn - 1) / bn);
     const int skt = sk_tiles_for(tiles, (K + BK - 1) / BK, sms, mt);
     if (skt > 0 && sk_ready()) {
@@ -1875,16 +1867,12 @@ static int gemm_call(const void* A, const void* B, void* C, const void* bias, co
   // the stream-K workspace is shared: a launch on another stream than the previous user waits for that one
   if (sk_on && g_sk_stream != st && g_sk_epoch > 1) cudaStreamWaitEvent(st, g_sk_event, 0);
   int rc;
-  if (split > 1) {
-    switch (bn * 10 + split) {
-      case 642: return launch_split<64, 2>(ta, tb, p, st);
-      case 644: return launch_split<64, 4>(ta, tb, p, st);
-      case 1282: return launch_split<128, 2>(ta, tb, p, st);
-      case 1284: return launch_split<128, 4>(ta, tb, p, st);
-      case 1922: return launch_split<192, 2>(ta, tb, p, st);
-      case 1924: return launch_split<192, 4>(ta, tb, p, st);
-      case 2562: return launch_split<256, 2>(ta, tb, p, st);
-      case 2564: return launch_split<256, 4>(ta, tb, p, st);
+  if (small) {
+    switch (bn) {
+      case 64: return launch_small<64>(ta, tb, p, st);
+      case 128: return launch_small<128>(ta, tb, p, st);
+      case 192: return launch_small<192>(ta, tb, p, st);
+      case 256: return launch_small<256>(ta, tb, p, st);
       default: return -4;
     }
   }

@@ -1,5 +1,4 @@
-"""GEMMs whose K loop is shared by a cluster: every width and split, tails, layouts, epilogues; and the shapes that choose
-one by themselves."""
+"""GEMMs with one tile per CTA: every width, tails, layouts, epilogues; and the shapes that choose one by themselves."""
 import pytest
 import torch
 
@@ -19,11 +18,10 @@ def _close(got, want, K):
     return ((got.double() - want).abs().max() / scale).item() < 2 ** -8 + K * 2 ** -24
 
 
-@pytest.mark.parametrize("split", [2, 4])
 @pytest.mark.parametrize("bn", [64, 128, 192, 256])
 @pytest.mark.parametrize("layout", ["kk", "k_mn", "mn_mn"])
 @pytest.mark.parametrize("M,N,K", [(128, 256, 512), (72, 136, 520), (264, 8, 1000), (136, 328, 3424)])
-def test_every_split(M, N, K, layout, bn, split):
+def test_every_width(M, N, K, layout, bn):
     from multimodal_training_b200.ops import functional as F
     from multimodal_training_b200.ops import native as nv
     torch.manual_seed(M + N + K)
@@ -35,7 +33,7 @@ def test_every_split(M, N, K, layout, bn, split):
     f32_old = f32.clone()
     try:
         nv.lib().mmt_gemm_force_bn(bn)
-        nv.lib().mmt_gemm_force_split(split)
+        nv.lib().mmt_gemm_force_small(1)
         plain = F.gemm(a, b, **kw)
         full = F.gemm(a, b, bias=bias, residual=res, alpha=0.5, **kw)
         gelu = F.gemm(a, b, bias=bias, act=1, **kw)
@@ -44,7 +42,7 @@ def test_every_split(M, N, K, layout, bn, split):
         again = F.gemm(a, b, **kw)
     finally:
         nv.lib().mmt_gemm_force_bn(0)
-        nv.lib().mmt_gemm_force_split(-1)
+        nv.lib().mmt_gemm_force_small(-1)
     assert nv.get_error()[0] == 0
     assert torch.equal(plain, again)
     assert _close(plain, want, K)
@@ -61,3 +59,24 @@ def test_shapes_that_do_not_fill_the_gpu(M, N, K):
     torch.manual_seed(M + N + K)
     A, B, kw, a, b = _operands(M, N, K, "kk")
     assert _close(F.gemm(a, b), A.double() @ B.double().t(), K)
+
+
+@pytest.mark.parametrize("bn", [64, 128, 192, 256])
+def test_one_tile_per_cta_has_the_bits_of_the_persistent_kernel(bn):
+    from multimodal_training_b200.ops import functional as F
+    from multimodal_training_b200.ops import native as nv
+    torch.manual_seed(bn)
+    A, B, kw, a, b = _operands(264, 328, 1000, "kk")
+    bias, res = torch.randn(328, device="cuda").bfloat16(), torch.randn(264, 328, device="cuda").bfloat16()
+    got = []
+    try:
+        nv.lib().mmt_gemm_force_bn(bn)
+        for small in (0, 1):
+            nv.lib().mmt_gemm_force_small(small)
+            acc = res.clone()
+            F.gemm(a, b, out=acc, accumulate=True, **kw)
+            got.append((F.gemm(a, b, bias=bias, residual=res, **kw), F.gemm(a, b, bias=bias, act=1, **kw), acc))
+    finally:
+        nv.lib().mmt_gemm_force_bn(0)
+        nv.lib().mmt_gemm_force_small(-1)
+    assert all(torch.equal(x, y) for x, y in zip(*got))
