@@ -37,10 +37,10 @@ using namespace attn;
 //     A tile skips the blocks outside its own visible range (packed sequences, causal).
 //   * P never touches shared memory: the softmax threads write it as packed bf16 pairs over the first 64
 //     columns of the S tile they have just read (tcgen05.st), and PV takes it as the tensor-memory A operand.
-//   * A thread reads its 128 scores ONCE, into registers, and maximum, exponentials and sum run from there with
-//     packed fp32 pairs: per 128 x 128 tile the exponentials alone need 1024 cycles of an SM (16 per cycle), the MMAs
+//   * A thread reads its 128 scores into registers once (the last 32 twice) and maximum, exponentials and sum run from
+//     there, the scaling on packed fp32 pairs: per 128 x 128 tile the exponentials alone need 1024 cycles of an SM (16 per cycle), the MMAs
 //     640 (head_dim 80), so everything else has to fit beside them.  Reading
-//     the scores twice, one wait per 32 columns: 2.00 ms for one image of 16384 patches (16 heads of 80), now 1.53 ms.
+//     the scores twice, one wait per 32 columns: 2.00 ms for one image of 16384 patches (16 heads of 80), now 1.59 ms.
 //   * O stays in tensor memory for the whole KV loop (PV accumulates).  The running maximum is lazy: O and l
 //     are rescaled only when a row's maximum grew by more than 2^8 since the value in use, which after the
 //     first tiles is rare; the rescale is a tensor-memory read-modify-write by the row's own thread, safe

@@ -83,7 +83,7 @@ __global__ void attn_group_reduce_kernel(const float* __restrict__ ws_dk, const 
 //     bubbles in the tensor pipe, the more so the narrower they are.
 //   * sixteen softmax warps (four per scheduler): with eight, the latency of a block's chain was not covered.
 // Measured (delta, dK/dV and dQ together, from two barriers and loads in the softmax warps to this): one image of 16384
-// patches, 16 heads of 80: 8.28 -> 5.5 ms; one causal sequence of 6144 tokens, 40 / 8 heads of 128: 2.09 -> 1.50 ms.
+// patches, 16 heads of 80: 8.28 -> 5.6 ms; one causal sequence of 6144 tokens, 40 / 8 heads of 128: 2.09 -> 1.50 ms.
 // What bounds it now: the chain MMA -> tcgen05.ld -> exponentials -> tcgen05.st of a block with two score stages; the
 // N = 64 products take about 70 cycles each (they read 6 KB of shared memory).
 // Tensor memory: stage s at columns 128 s: S^T [0,64) (P^T over [0,32)), dP^T [64,128) (dS^T over [64,96));
