@@ -566,17 +566,18 @@ __global__ void colsum_partial_kernel(const bf16* __restrict__ x, float* __restr
 // stats: per row, max over the local vocab shard, sum exp(l - max), and the target logit if the
 // label falls into [vocab_lo, vocab_lo + V) (else 0).
 // grad (in place): l <- (exp(l - gmax) / gsum - [label == col]) * scale for valid rows, 0 otherwise.
+// The logits may hold compacted rows (compact_labels_kernel): the statistics stay in the order of the caller's rows.
 // ----------------------------------------------------------------------------
 constexpr int kCeThreads = 512;
 
 __global__ void __launch_bounds__(kCeThreads) ce_stats_kernel(const bf16* __restrict__ logits,
                                                              const long* __restrict__ labels, float* __restrict__ omax,
                                                              float* __restrict__ osum, float* __restrict__ otgt, int V,
-                                                             long ld, long vocab_lo) {
+                                                             long ld, long vocab_lo, const long* __restrict__ pos,
+                                                             long base) {
   grid_dependency_sync();
   __shared__ float red[32];
   const long row = blockIdx.x;
-  const bf16* l = logits + row * ld;
   const int nvec = V >> 3;
   if (labels[row] < 0) {            // an ignored row takes no part in the loss; its statistics only have to be finite
     if (threadIdx.x == 0) {
@@ -586,6 +587,7 @@ __global__ void __launch_bounds__(kCeThreads) ce_stats_kernel(const bf16* __rest
     }
     return;
   }
+  const bf16* l = logits + (pos ? pos[row] - base : row) * ld;
   float m = -INFINITY, s = 0.f;
   for (int c = threadIdx.x; c < nvec; c += kCeThreads) {
     float v[8];
@@ -615,15 +617,16 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* __restrict__ 
                                                             const float* __restrict__ gmax,
                                                             const float* __restrict__ gsum,
                                                             const float* __restrict__ scale_ptr, int V, long ld,
-                                                            long vocab_lo, const int* __restrict__ cnt, int base) {
+                                                            long vocab_lo, const int* __restrict__ cnt,
+                                                            const long* __restrict__ src, long base) {
   grid_dependency_sync();
   const long row = blockIdx.x;
   bf16* l = logits + row * ld;
   const int nvec = V >> 3;
   if (cnt) {
-    // compacted rows: those behind the last valid one are not read again, except that the weight gradient's last block
-    // of 64 rows (the first one if there is no valid row) has to end in zeros
-    const int n = max(*cnt - base, 0);
+    // compacted rows: those behind the last one are not read again, except that the weight gradient's last block of 64
+    // rows (the first one if there is none) has to end in zeros
+    const int n = *cnt;
     if (row >= n && row >= max((n + 63) / 64 * 64, 64)) return;
   }
   const long lab_g = labels[row];
@@ -634,8 +637,9 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* __restrict__ 
   }
   const long lab = lab_g - vocab_lo;
   const float scale = *scale_ptr;
-  const float m = gmax[row];
-  const float inv = 1.f / gsum[row];
+  const long st = src ? src[row] - base : row;
+  const float m = gmax[st];
+  const float inv = 1.f / gsum[st];
   for (int c = threadIdx.x; c < nvec; c += kCeThreads) {
     float v[8];
     load8(l + c * 8, v);
@@ -650,41 +654,57 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* __restrict__ 
 }
 
 // ----------------------------------------------------------------------------
-// Rows with a label, in order: src[j] = the j-th such row and its label, -1 and -1 behind the last; pos[t] = j or -1;
-// *count = their number.  One CTA: a few thousand labels are a few microseconds, and nothing waits for the host.
+// Blocks of rows with a label.  The rows are cut into chunks and a chunk into blocks of kLabelBlock; a block in which no
+// row has a label is dropped and the others move to the front of their chunk, in order and whole.
+//   src[j] = row that place j takes, lab[j] = its label; -1 and -1 behind a chunk's last place
+//   pos[t] = place of row t, or -1;   count[i] = places of chunk i that are taken
+// A block is one k-block of the weight gradient's GEMM and chunks are never joined, so that GEMM adds what it would add
+// without this, in the same groups and order, less k-blocks of zeros: its bits stay the same.  (Moving single rows
+// together saves a little more work where labels are scattered, and adds in another order.)
+// One CTA per chunk: a few thousand labels are a few microseconds, and nothing waits for the host.
 // ----------------------------------------------------------------------------
 constexpr int kCompactThreads = 1024;
-__global__ void __launch_bounds__(kCompactThreads) compact_labels_kernel(const long* __restrict__ labels, long n,
+constexpr int kLabelBlock = 64;
+__global__ void __launch_bounds__(kCompactThreads) compact_labels_kernel(const long* __restrict__ labels, long n, long chunk,
                                                                         long* __restrict__ src, long* __restrict__ lab,
                                                                         long* __restrict__ pos, int* __restrict__ count) {
   grid_dependency_sync();
-  __shared__ int warp_total[32];
+  constexpr int kBlocks = kCompactThreads / kLabelBlock, kWarpsPerBlock = kLabelBlock / 32;
+  __shared__ int labelled[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int base = 0;
-  for (long t0 = 0; t0 < n; t0 += kCompactThreads) {
+  const int mine = threadIdx.x / kLabelBlock;
+  const long c0 = blockIdx.x * chunk, c1 = min(c0 + chunk, n);
+  long place = c0;                                   // first place that is still free
+  for (long t0 = c0; t0 < c1; t0 += kCompactThreads) {
     const long t = t0 + threadIdx.x;
-    const long l = t < n ? labels[t] : -1;
-    const unsigned ballot = __ballot_sync(0xffffffffu, l >= 0);
-    if (lane == 0) warp_total[warp] = __popc(ballot);
+    const long l = t < c1 ? labels[t] : -1;
+    const bool any = __any_sync(0xffffffffu, l >= 0);
+    if (lane == 0) labelled[warp] = any;
     __syncthreads();
     int before = 0, total = 0;
+    bool keep = false;
 #pragma unroll
-    for (int w = 0; w < 32; ++w) {
-      const int v = warp_total[w];
-      before += w < warp ? v : 0;
+    for (int b = 0; b < kBlocks; ++b) {
+      int v = 0;
+#pragma unroll
+      for (int w = 0; w < kWarpsPerBlock; ++w) v |= labelled[b * kWarpsPerBlock + w];
+      before += b < mine ? v : 0;
       total += v;
+      if (b == mine) keep = v != 0;
     }
-    const int j = base + before + __popc(ballot & ((1u << lane) - 1u));
-    if (t < n) pos[t] = l >= 0 ? j : -1;
-    if (l >= 0) {
-      src[j] = t;
+    // a chunk's last block may be shorter than the others; its places behind the last row stay empty
+    const long j = place + (long)before * kLabelBlock + threadIdx.x % kLabelBlock;
+    if (t < c1) pos[t] = keep ? j : -1;
+    if (keep && j < c1) {
+      src[j] = t < c1 ? t : -1;
       lab[j] = l;
     }
-    base += total;
+    place += (long)total * kLabelBlock;
     __syncthreads();
   }
-  for (long j = base + threadIdx.x; j < n; j += kCompactThreads) src[j] = lab[j] = -1;
-  if (threadIdx.x == 0) *count = base;
+  const long end = min(place, c1);
+  for (long j = end + threadIdx.x; j < c1; j += kCompactThreads) src[j] = lab[j] = -1;
+  if (threadIdx.x == 0) count[blockIdx.x] = (int)(end - c0);
 }
 
 // ----------------------------------------------------------------------------
@@ -1002,28 +1022,28 @@ int mmt_colsum(const void* x, void* out, float* scratch, long rows, int cols, lo
 }
 
 int mmt_ce_stats(const void* logits, const long* labels, float* omax, float* osum, float* otgt, long rows, int V,
-                 long ld, long vocab_lo, void* stream) {
+                 long ld, long vocab_lo, const long* pos, long base, void* stream) {
   if (V % 8 || ld % 8) return -2;
   if (rows == 0) return 0;
-  launch_dependent(ce_stats_kernel, (unsigned)rows, kCeThreads, 0, ST(stream),
-                     CBF(logits), labels, omax, osum, otgt, V, ld,
-                                                                vocab_lo);
+  launch_dependent(ce_stats_kernel, (unsigned)rows, kCeThreads, 0, ST(stream), CBF(logits), labels, omax, osum, otgt, V, ld,
+                   vocab_lo, pos, base);
   return (int)cudaGetLastError();
 }
-// cnt (optional): rows [0, *cnt - base) are valid, the rest is not needed (see ce_grad_kernel).
+// cnt (optional): rows [0, *cnt) are needed (see ce_grad_kernel); row r has its statistics at src[r] - base.
 int mmt_ce_grad(void* logits, const long* labels, const float* gmax, const float* gsum, const float* scale_ptr,
-                long rows, int V, long ld, long vocab_lo, const int* cnt, int base, void* stream) {
+                long rows, int V, long ld, long vocab_lo, const int* cnt, const long* src, long base, void* stream) {
   if (V % 8 || ld % 8) return -2;
   if (rows == 0) return 0;
-  launch_dependent(ce_grad_kernel, (unsigned)rows, kCeThreads, 0, ST(stream),
-                     BF(logits), labels, gmax, gsum, scale_ptr, V, ld,
-                                                               vocab_lo, cnt, base);
+  launch_dependent(ce_grad_kernel, (unsigned)rows, kCeThreads, 0, ST(stream), BF(logits), labels, gmax, gsum, scale_ptr, V,
+                   ld, vocab_lo, cnt, src, base);
   return (int)cudaGetLastError();
 }
 
-int mmt_compact_labels(const long* labels, long n, long* src, long* lab, long* pos, int* count, void* stream) {
-  if (n < 0 || n > 0x7fffffffL) return -5;
-  return (int)launch_dependent(compact_labels_kernel, 1, kCompactThreads, 0, ST(stream), labels, n, src, lab, pos, count);
+int mmt_compact_labels(const long* labels, long n, long chunk, long* src, long* lab, long* pos, int* count, void* stream) {
+  if (n < 0 || chunk <= 0 || chunk > 0x7fffffffL) return -5;
+  if (n == 0) return 0;
+  return (int)launch_dependent(compact_labels_kernel, (unsigned)((n + chunk - 1) / chunk), kCompactThreads, 0, ST(stream),
+                               labels, n, chunk, src, lab, pos, count);
 }
 
 int mmt_adamw(void* p, const void* g, float* master, float* m, float* v, long n, long n_decay, float lr, float b1,

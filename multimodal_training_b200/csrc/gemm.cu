@@ -67,12 +67,12 @@ struct GemmParams {
   int group_m, tiles_n;           // raster: m-tiles per band (0 = all), number of n-tiles
   uint32_t mn_lbo, mn_sbo, mn_kstep;  // descriptor constants of MN-major tiles
   MmtErrorWord* ew;
-  // --- number of rows (cnt_k == 0) or length of K (cnt_k == 1) known on the device only: min(max(*cnt - cnt_base, 0), M or K).
+  // --- number of rows (cnt_k == 0) or length of K (cnt_k == 1) known on the device only: min(max(*cnt, 0), M or K).
   //     Rows: tiles beyond the last row are not computed, and the launch does nothing unless the count falls into one of
   //     its buckets (bit (rows - 1) / cnt_bucket of cnt_mask).  K: k-blocks beyond the count are not read; the rest of the
   //     last one has to hold zeros (also the first one when the count is 0).  nullptr: M and K are what they are.
   const int* cnt;
-  int cnt_base, cnt_k, cnt_bucket;
+  int cnt_k, cnt_bucket;
   uint32_t cnt_mask;
   int local_only;                 // no waits on other CTAs or peers: this launch may overlap its neighbours' ends
   // --- stream-K for the last partial wave: the final `sk_tiles` tiles are cut along K into gridDim.x equal runs of
@@ -778,7 +778,7 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   grid_dependency_wait();
   int m_rows = p.M, k_len = p.K;
   if (p.cnt) {
-    const int n = warp_uniform(min(max(*p.cnt - p.cnt_base, 0), p.cnt_k ? p.K : p.M));
+    const int n = warp_uniform(min(max(*p.cnt, 0), p.cnt_k ? p.K : p.M));
     if (p.cnt_k) k_len = max(n, 1);
     else m_rows = n > 0 && ((p.cnt_mask >> ((n - 1) / p.cnt_bucket)) & 1u) ? n : 0;
   }
@@ -1626,7 +1626,7 @@ extern "C" void mmt_gemm_set_comm(const MmtGemmComm* c) { g_comm = c; }
 // A count that only the device knows (GemmParams::cnt) and, for a count of rows, the tile of this launch.
 struct GemmCount {
   const int* cnt;
-  int base, is_k, bucket;
+  int is_k, bucket;
   uint32_t mask;
   int mt, bn;
 };
@@ -1735,7 +1735,6 @@ static int gemm_call(const void* A, const void* B, void* C, const void* bias, co
   p.mn_lbo = g_mn_lbo; p.mn_sbo = g_mn_sbo; p.mn_kstep = g_mn_kstep;
   p.ew = mmt_error_word();
   p.cnt = count ? count->cnt : nullptr;
-  p.cnt_base = count ? count->base : 0;
   p.cnt_k = count ? count->is_k : 0;
   p.cnt_bucket = count ? count->bucket : 1;
   p.cnt_mask = count ? count->mask : 0;
@@ -1900,15 +1899,14 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
                    nullptr, stream);
 }
 
-// The same product over the first min(max(*cnt - base, 0), M) rows of A and C (is_k == 0; later rows of C are undefined)
+// The same product over the first min(max(*cnt, 0), M) rows of A and C (is_k == 0; later rows of C are undefined)
 // or over that many of the K rows of MN-major A and B (is_k == 1; see GemmParams::cnt for the zeros it needs).  The host
 // does not know the count, and which tile is best depends on it: a row count is cut into up to 32 buckets, and every
 // tile that is the best of some bucket is launched; the launches that the count does not belong to return at once.
 extern "C" int mmt_gemm_bf16_counted(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                                     int a_mn, int b_mn, int accumulate, const int* cnt, int base, int is_k,
-                                     void* stream) {
+                                     int a_mn, int b_mn, int accumulate, const int* cnt, int is_k, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  GemmCount c = {cnt, base, is_k, 1, 0u, 0, 0};
+  GemmCount c = {cnt, is_k, 1, 0u, 0, 0};
   if (is_k)
     return gemm_call(A, B, C, nullptr, nullptr, M, N, K, lda, ldb, ldc, 0, a_mn, b_mn, 0, accumulate, 0, 1.f, 0, &c, stream);
   read_env_once();

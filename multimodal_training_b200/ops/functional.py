@@ -79,9 +79,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     return out
 
 
-def _gemm_counted(a, b, out, count: torch.Tensor, base: int, *, of_k: bool = False, a_mn: bool = False,
+def _gemm_counted(a, b, out, count: torch.Tensor, *, of_k: bool = False, a_mn: bool = False,
                   b_mn: bool = False, accumulate: bool = False) -> None:
-    """:func:`gemm` over as many rows (``of_k``: as many k) as ``count[0] - base``, a number on the device.  Rows of
+    """:func:`gemm` over as many rows (``of_k``: as many k) as ``count[0]``, a number on the device.  Rows of
     ``out`` behind them are undefined; with ``of_k`` the last block of 64 has to be filled up with zeros."""
     K, M = a.shape if a_mn else a.shape[::-1]
     N = b.shape[1] if b_mn else b.shape[0]
@@ -89,7 +89,7 @@ def _gemm_counted(a, b, out, count: torch.Tensor, base: int, *, of_k: bool = Fal
     if M == 0 or K == 0:
         return
     nv.call("mmt_gemm_bf16_counted", a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-            out.stride(0), int(a_mn), int(b_mn), int(accumulate), count.data_ptr(), base, int(of_k), nv.stream())
+            out.stride(0), int(a_mn), int(b_mn), int(accumulate), count.data_ptr(), int(of_k), nv.stream())
 
 
 def _write_param_grad(p: torch.Tensor, compute) -> torch.Tensor | None:
@@ -446,33 +446,35 @@ class _LMHeadCEFn(torch.autograd.Function):
             else:
                 dw = mg
                 acc0 = bool(getattr(weight, "grad_written", False))
-        # Rows without a label (image tokens, prompts, the last token of a sample) have no loss and no gradient: the rows
-        # that have one are moved together and the chunks below stop behind the last of them.  Their number stays on the
-        # device.  (Label smoothing works on plain tensors of all rows.)  Half of a sample's rows are image tokens in the
-        # 7B configuration, two thirds in the 32B one: text steps 16.6 -> 14.5 and 57.6 -> 44.2 ms.
-        x, labs, ok, dx, count, pos = hidden, labels, valid, dhidden, None, None
+        # Rows without a label (image tokens, prompts, the last token of a sample) have no loss and no gradient: blocks of
+        # rows that have none are left out, the others of a chunk move to its front, and the products below stop behind
+        # the last of them.  Their number stays on the device.  (Label smoothing works on plain tensors of all rows.)
+        # Half of a sample's rows are image tokens in the 7B configuration, two thirds in the 32B one.
+        x, labs, dx, count, src, pos = hidden, labels, dhidden, None, None, None
         if smoothing == 0.0 and T > 0:
             src, labs, pos = torch.empty(3, T, device=dev, dtype=torch.int64)
-            count = torch.empty(1, device=dev, dtype=torch.int32)
-            lab64 = _c(labels.to(torch.int64))
-            nv.call("mmt_compact_labels", lab64.data_ptr(), T, src.data_ptr(), labs.data_ptr(), pos.data_ptr(),
-                    count.data_ptr(), nv.stream())
+            count = torch.empty((T + chunk_rows - 1) // chunk_rows, device=dev, dtype=torch.int32)
+            labels = _c(labels.to(torch.int64))
+            nv.call("mmt_compact_labels", labels.data_ptr(), T, min(chunk_rows, T), src.data_ptr(), labs.data_ptr(),
+                    pos.data_ptr(), count.data_ptr(), nv.stream())
             x = gather_rows_raw(hidden, src)
             dx = torch.empty_like(hidden)
-            ok = labs >= 0
         for c0 in range(0, T, chunk_rows):
             c1 = min(T, c0 + chunk_rows)
             rows = c1 - c0
             h = x[c0:c1]
-            lab = labs[c0:c1]
+            lab = labels[c0:c1]
             logits = ws[:rows]
+            n_rows = None if count is None else count[c0 // chunk_rows:]
             if count is not None:
-                _gemm_counted(h, weight, logits, count, c0)
+                _gemm_counted(h, weight, logits, n_rows)
             else:
                 gemm(h, weight, out=logits)
+            # statistics and losses in the order of `labels`, logits and their gradient in that of `labs`
             st = torch.empty(3, rows, device=dev, dtype=torch.float32)
             nv.call("mmt_ce_stats", logits.data_ptr(), lab.data_ptr(), st[0].data_ptr(), st[1].data_ptr(),
-                    st[2].data_ptr(), rows, V, logits.stride(0), vocab_lo, nv.stream())
+                    st[2].data_ptr(), rows, V, logits.stride(0), vocab_lo, nv.ptr(pos if pos is None else pos[c0:]), c0,
+                    nv.stream())
             if group is not None and torch.distributed.get_world_size(group) > 1:
                 lmax = st[0].clone()
                 _all_reduce(st[0], ReduceOp.MAX, group)
@@ -484,23 +486,24 @@ class _LMHeadCEFn(torch.autograd.Function):
                 zsum = logits.sum(-1, dtype=torch.float32)
                 _all_reduce(zsum, ReduceOp.SUM, group)
                 row_loss = (torch.log(st[1]) + st[0] - (1.0 - smoothing) * st[2] - smoothing * zsum / vocab_total) \
-                    * ok[c0:c1]
+                    * valid[c0:c1]
             else:
-                row_loss = (torch.log(st[1]) + st[0] - st[2]) * ok[c0:c1]
+                row_loss = (torch.log(st[1]) + st[0] - st[2]) * valid[c0:c1]
             loss_sum += row_loss.sum()
-            nv.call("mmt_ce_grad", logits.data_ptr(), lab.data_ptr(), st[0].data_ptr(), st[1].data_ptr(),
-                    inv.data_ptr(), rows, V, logits.stride(0), vocab_lo, nv.ptr(count), c0, nv.stream())
+            nv.call("mmt_ce_grad", logits.data_ptr(), labs[c0:].data_ptr(), st[0].data_ptr(), st[1].data_ptr(),
+                    inv.data_ptr(), rows, V, logits.stride(0), vocab_lo, nv.ptr(n_rows),
+                    nv.ptr(src if src is None else src[c0:]), c0, nv.stream())
             if smoothing > 0.0:
-                scale = (inv[0] * ok[c0:c1]).to(logits.dtype)                       # [rows]
+                scale = (inv[0] * valid[c0:c1]).to(logits.dtype)                       # [rows]
                 logits.sub_((smoothing / vocab_total) * scale.unsqueeze(1))
                 local = lab - vocab_lo
-                mine = (local >= 0) & (local < V) & ok[c0:c1]
+                mine = (local >= 0) & (local < V) & valid[c0:c1]
                 logits.view(-1).index_add_(0, (torch.arange(rows, device=dev) * logits.stride(0)
                                                + local.clamp(0, V - 1))[mine], (smoothing * scale)[mine])
             if count is not None:
-                _gemm_counted(logits, weight, dx[c0:c1], count, c0, b_mn=True)
+                _gemm_counted(logits, weight, dx[c0:c1], n_rows, b_mn=True)
                 if need_w:
-                    _gemm_counted(logits, h, dw, count, c0, of_k=True, a_mn=True, b_mn=True, accumulate=acc0 or c0 > 0)
+                    _gemm_counted(logits, h, dw, n_rows, of_k=True, a_mn=True, b_mn=True, accumulate=acc0 or c0 > 0)
                 continue
             gemm(logits, weight, b_mn=True, out=dx[c0:c1])
             if need_w:

@@ -67,3 +67,45 @@ def test_weight_gradient_accumulates_over_steps():
             total += z.T @ h[:n].double() / n
     # every accumulation rounds to bf16
     assert ((w.main_grad.double() - total).norm() / total.norm()).item() < 1.5e-2
+
+
+@pytest.mark.parametrize("T,chunk", [(70, 4096), (300, 128), (1025, 512), (1500, 4096), (2000, 1000), (333, 100)])
+@pytest.mark.parametrize("kind", ["none", "1", "63", "65", "half", "tail", "all", "image"])
+@pytest.mark.parametrize("written", [False, True])
+def test_rows_left_out_change_no_bit(T, chunk, kind, written):
+    """The same chunks over all rows, one kernel at a time: loss and gradients must not depend on what is left out."""
+    from multimodal_training_b200.ops import functional as F
+    from multimodal_training_b200.ops import native as nv
+    g = torch.Generator().manual_seed(T + 1)
+    H, V = 256, 1544
+    h = torch.randn(T, H, generator=g).cuda().bfloat16().requires_grad_()
+    w = torch.nn.Parameter((torch.randn(V, H, generator=g) * 0.1).cuda().bfloat16())
+    w.main_grad = (torch.randn(V, H, generator=g) * 1e-3).cuda().bfloat16()
+    w.grad_written = written
+    if kind == "image":                         # one run of rows without a label
+        labels = torch.randint(0, V, (T,), generator=g)
+        labels[T // 4 + 7:T // 4 + 7 + T // 2] = -100
+    else:
+        labels = _labels(kind, T, V, g)
+    labels = labels.cuda()
+    want_w, want_h = w.main_grad.clone(), torch.empty_like(h)
+    inv = (1.0 / (labels >= 0).sum().float().clamp(min=1.0)).reshape(1)
+    want = torch.zeros((), device="cuda")
+    for c0 in range(0, T, chunk):
+        hc, lab = h.detach()[c0:c0 + chunk], labels[c0:c0 + chunk]
+        rows = hc.shape[0]
+        logits = F.gemm(hc, w.detach())
+        st = torch.empty(3, rows, device="cuda")
+        nv.call("mmt_ce_stats", logits.data_ptr(), lab.data_ptr(), st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(),
+                rows, V, V, 0, None, 0, nv.stream())
+        want += ((torch.log(st[1]) + st[0] - st[2]) * (lab >= 0)).sum()
+        nv.call("mmt_ce_grad", logits.data_ptr(), lab.data_ptr(), st[0].data_ptr(), st[1].data_ptr(), inv.data_ptr(), rows,
+                V, V, 0, None, None, 0, nv.stream())
+        F.gemm(logits, w.detach(), b_mn=True, out=want_h[c0:c0 + chunk])
+        F.gemm(logits, hc, a_mn=True, b_mn=True, out=want_w, accumulate=written or c0 > 0)
+    loss = F.lm_head_cross_entropy(h, w, labels, chunk_rows=chunk)
+    loss.backward()
+    assert nv.get_error()[0] == 0
+    assert torch.equal(loss.detach(), want * inv[0])
+    assert torch.equal(h.grad, want_h)
+    assert torch.equal(w.main_grad, want_w)
