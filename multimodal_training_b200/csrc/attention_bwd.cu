@@ -12,6 +12,7 @@
 // Every tile is fetched as 64-column TMA boxes that serve as K-major or MN-major operands, so Q, K, V and dO
 // need no transposes.  Details at the kernels.
 #include "attention_common.cuh"
+#include "block_loop.h"
 
 namespace {
 using namespace attn;
@@ -283,14 +284,16 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
     const uint32_t lane_addr = ((uint32_t)(q4 * 32) << 16);
     const float sl2 = p.scale * LOG2E;
     const float2 sl2_2 = make_float2(sl2, sl2), scale_2 = make_float2(p.scale, p.scale);
-    bool ok = true;
-    for (int it = 0; it < n_iter; ++it) {
+    const auto arrived = [&](int it) {
+      return __all_sync(0xffffffffu, mbar_wait(&row_full[it % kRing], (it / kRing) & 1, p.ew, 752) &&
+                                         mbar_wait(&s_full[it & 1], (it >> 1) & 1, p.ew, 750)) != 0;
+    };
+    // all warps of the quadrant have read their columns (P^T / dS^T overwrite them)
+    const auto together = [&] { quadrant_bar_sync<kSoftWarps / 4>(q4); };
+    const auto work = [&](int it) {
       const int s = it & 1;
       const int buf = it % kRing;
       const float* rowv = sRow + buf * 4 * BQ2;
-      ok = __all_sync(0xffffffffu, mbar_wait(&row_full[buf], (it / kRing) & 1, p.ew, 752) &&
-                                       mbar_wait(&s_full[s], (it >> 1) & 1, p.ew, 750));
-      if (!ok) break;
       tc_fence_after();
       const uint32_t st = tmem_base + lane_addr + (uint32_t)(s * 128);
       uint32_t r_s[16], r_dp[16];
@@ -301,7 +304,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
       const float4* dl_v = reinterpret_cast<const float4*>(rowv + 3 * BQ2 + part * 16);
       tmem_wait_ld();
       tc_fence_before();
-      quadrant_bar_sync<kSoftWarps / 4>(q4);       // all warps of the quadrant have read their columns (P^T / dS^T overwrite them)
+      together();
       tc_fence_after();
       uint32_t pk_p[8], pk_ds[8];
 #pragma unroll
@@ -337,7 +340,8 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&pds_full[s]);
-    }
+    };
+    bool ok = for_blocks_in_step(n_iter, arrived, work, together);
     // epilogue: thread = kv row; of a quadrant's four warps two write dK and two dV, alternate chunks of 16 columns
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(done, 0, p.ew, 751));
     tc_fence_after();
@@ -544,12 +548,14 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     const float2 sl2_2 = make_float2(sl2, sl2), scale_2 = make_float2(p.scale, p.scale);
     const float2 lse_2 = make_float2(-lse_l2, -lse_l2), delta_2 = make_float2(-delta, -delta);
-    bool ok = true;
-    for (int it = 0; it < n_iter; ++it) {
+    const auto arrived = [&](int it) {
+      return __all_sync(0xffffffffu, mbar_wait(&s_full[it & 1], (it >> 1) & 1, p.ew, 780)) != 0;
+    };
+    // all warps of the quadrant have read their dP columns before dS overwrites them
+    const auto together = [&] { quadrant_bar_sync<kSoftWarps / 4>(q4); };
+    const auto work = [&](int it) {
       const int s = it & 1;
       const int kvb = kv_lo + it * BQ2 + part * 16;          // first kv row of this warp's 16 columns
-      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[s], (it >> 1) & 1, p.ew, 780));
-      if (!ok) break;
       tc_fence_after();
       const uint32_t st = tmem_base + lane_addr + (uint32_t)(s * 128);
       uint32_t r_s[16], r_dp[16];
@@ -558,7 +564,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const bool full = __all_sync(0xffffffffu, kvb >= lo && kvb + 16 <= hi2);
       tmem_wait_ld();
       tc_fence_before();
-      quadrant_bar_sync<kSoftWarps / 4>(q4);       // all warps of the quadrant have read their dP columns before dS overwrites them
+      together();
       tc_fence_after();
       uint32_t pk_ds[8];
 #pragma unroll
@@ -579,7 +585,8 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ds_full[s]);
-    }
+    };
+    bool ok = for_blocks_in_step(n_iter, arrived, work, together);
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(done, 0, p.ew, 781));
     tc_fence_after();
     // epilogue: the warps of a lane quadrant split the head's columns in 16-column chunks
