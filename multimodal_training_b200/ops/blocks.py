@@ -252,13 +252,16 @@ class _LocalBlockFn(torch.autograd.Function):
 def local_block(x: torch.Tensor, spec: BlockSpec, cos: torch.Tensor, sin: torch.Tensor, seq: SeqInfo, params: tuple,
                 recompute: bool = True, keep_elementwise: bool = False):
     """``params`` = (ln1_w, qkv_w, qkv_b, proj_w, proj_b, ln2_w, gate_up_w, gate_up_b, down_w, down_b); biases may
-    be None.  x is [T, C] bf16 on the GPU; the result has the same shape.  cos and sin are [T, head_dim] fp32.
-    ``recompute``: keep only the block input and rebuild everything in backward (activation checkpointing); else keep
-    the GEMM / attention results and, with ``keep_elementwise``, the normalised inputs and the SwiGLU output as well."""
+    be None.  x is [T, C] bf16 on the GPU; the result has the same shape.  cos and sin are [T, head_dim] fp32; ``seq`` is
+    a :class:`SeqInfo` or a plain list of sequence boundaries.  ``recompute``: keep only the block input and rebuild
+    everything in backward (activation checkpointing); else keep the GEMM / attention results and, with
+    ``keep_elementwise``, the normalised inputs and the SwiGLU output as well."""
     assert x.dim() == 2
     for t in (cos, sin):         # the kernels get their addresses
         assert t.dtype == torch.float32 and t.is_contiguous() and t.device == x.device
         assert t.numel() >= x.shape[0] * spec.head_dim, (t.shape, x.shape, spec.head_dim)
+    if not isinstance(seq, SeqInfo):
+        seq = SeqInfo.from_list(list(seq), x.device)
     level = 2 if recompute or not torch.is_grad_enabled() else (0 if keep_elementwise else 1)
     return _LocalBlockFn.apply(x, spec, cos, sin, seq, level, *params)
 

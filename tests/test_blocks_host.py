@@ -49,3 +49,10 @@ def test_tables_of_the_wrong_kind_are_refused(block):
         with pytest.raises(AssertionError):
             block(sin=t)
     block(cos=torch.ones(40, 16), sin=torch.ones(40, 16))          # tables of a longer batch
+
+
+def test_sequence_boundaries_as_a_plain_list(block):
+    seq = block(seq=[0, 10, 24])[4]
+    assert isinstance(seq, SeqInfo) and seq.host == [0, 10, 24]
+    given = SeqInfo.from_list([0, 24], "cpu")
+    assert block(seq=given)[4] is given
