@@ -23,6 +23,7 @@ with communication inside (Ulysses layers, tensor-parallel layers) and as the or
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 
 import torch
@@ -113,7 +114,6 @@ def _linear_bwd(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, b) -> torch.
 # Native calls: csrc/block.cu takes one array of 64-bit words (addresses, sizes, flags) in this order
 # --------------------------------------------------------------------------------------
 _N_WORDS = 10 + 6 + 10 + 10 + 10 + 1 + 2 + 4 + 3 + 1
-_Words = ctypes.c_int64 * _N_WORDS
 nv.declare("mmt_block_words", nv.c_int, [])
 nv.declare("mmt_block_fwd", nv.c_int, [nv._P, nv.c_float, nv.c_float, nv._P])
 nv.declare("mmt_block_rebuild", nv.c_int, [nv._P, nv.c_float, nv._P])
@@ -154,6 +154,17 @@ def _front_words(x, y: int, P, cos, sin, seq, s: BlockSpec, act: dict, inter: in
         0 if packs is None else packs.data_ptr(), 0 if packs is None else packs.shape[0]]
 
 
+@functools.lru_cache(maxsize=None)
+def _words_type():
+    """The array type of the native calls.  They take its layout on trust and write its last word, so the library has to
+    agree on the length before the first of them."""
+    n = nv.lib().mmt_block_words()
+    if n != _N_WORDS:
+        raise RuntimeError(f"the kernel library's block calls take {n} words, this module builds {_N_WORDS}: rebuild it "
+                           "with `python -m multimodal_training_b200.csrc.build`")
+    return ctypes.c_int64 * _N_WORDS
+
+
 def _native_call(name: str, words, *args) -> None:
     nv.call(name, ctypes.addressof(words), *args, nv.stream())
     nv.launch_count += words[_N_WORDS - 1] - 1         # nv.call has counted one
@@ -178,7 +189,7 @@ class _LocalBlockFn(torch.autograd.Function):
         tmp, addr = _carve([sizes[k] for k in rest], x.device)
         act.update(zip(rest, addr))
         y = torch.empty_like(x)
-        words = _Words(*_front_words(x, y.data_ptr(), P, cos, sin, seq, s, act, inter))
+        words = _words_type()(*_front_words(x, y.data_ptr(), P, cos, sin, seq, s, act, inter))
         _native_call("mmt_block_fwd", words, s.eps, s.scale)
         ctx.save_for_backward(x, cos, sin, buf, *[p for p in params if p is not None])
         ctx.has = [p is not None for p in params]
@@ -228,7 +239,7 @@ class _LocalBlockFn(torch.autograd.Function):
                                 8 * s.n_q * T * s.head_dim if split else 0, 4 * parts], dev)
         if not split:
             addr[5] = 0
-        words = _Words(*_front_words(x, 0, P, cos, sin, seq, s, act, inter), *grads, acc, dy.data_ptr(), dx.data_ptr(),
+        words = _words_type()(*_front_words(x, 0, P, cos, sin, seq, s, act, inter), *grads, acc, dy.data_ptr(), dx.data_ptr(),
                        *addr)
         if level == 2:
             _native_call("mmt_block_fwd", words, s.eps, s.scale)

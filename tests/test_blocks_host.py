@@ -56,3 +56,16 @@ def test_sequence_boundaries_as_a_plain_list(block):
     assert isinstance(seq, SeqInfo) and seq.host == [0, 10, 24]
     given = SeqInfo.from_list([0, 24], "cpu")
     assert block(seq=given)[4] is given
+
+
+def test_library_and_module_agree_on_the_argument_array(monkeypatch):
+    from multimodal_training_b200.ops import native as nv
+    if not nv.available():
+        pytest.skip("the kernel library is not built")
+    blocks._words_type.cache_clear()
+    assert blocks._words_type()._length_ == nv.lib().mmt_block_words()
+    blocks._words_type.cache_clear()
+    monkeypatch.setattr(blocks, "_N_WORDS", blocks._N_WORDS + 1)         # a library of another layout
+    with pytest.raises(RuntimeError, match="rebuild"):
+        blocks._words_type()
+    blocks._words_type.cache_clear()
