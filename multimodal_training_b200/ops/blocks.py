@@ -228,8 +228,12 @@ class _LocalBlockFn(torch.autograd.Function):
                 acc |= int(written) << i
                 flat.append((p, mg, written))
             else:
-                g = torch.empty(p.shape, device=dev, dtype=p.dtype)
-                fresh.append((p, mg, g))
+                # no view of the flat buffer, or one with gaps: a dense array, which takes the values that are there
+                # along, since a sum that is rounded before it is added would be rounded twice
+                written = mg is not None and bool(getattr(p, "grad_written", False))
+                g = mg.contiguous() if written else torch.empty(p.shape, device=dev, dtype=p.dtype)
+                fresh.append((p, mg, g, written))
+                acc |= int(written) << i
                 grads.append(g.data_ptr())
         parts = 2 * nv.lib().mmt_rmsnorm_bwd_parts(T) * C + nv.lib().mmt_colsum_parts(T) * sum(
             b.shape[0] for b in (P[2], P[4], P[7], P[9]) if b is not None)
@@ -247,15 +251,15 @@ class _LocalBlockFn(torch.autograd.Function):
             _native_call("mmt_block_rebuild", words, s.eps)
         _native_call("mmt_block_bwd", words, s.scale)
         if T == 0:                                # no rows, no launches: gradients that nothing wrote are zero
-            for t in [mg for _, mg, written in flat if not written] + [g for _, _, g in fresh]:
+            for t in [mg for _, mg, w in flat if not w] + [g for _, _, g, w in fresh if not w]:
                 t.zero_()
         for p, _, _ in flat:
             p.grad_written = True
-        for p, mg, g in fresh:
+        for p, mg, g, _ in fresh:
             if mg is None:
                 p.grad = g if p.grad is None else p.grad + g
             else:
-                mg.copy_(mg + g if getattr(p, "grad_written", False) else g)
+                mg.copy_(g)
                 p.grad_written = True
         return (dx, None, None, None, None, None) + (None,) * len(ctx.has)
 
