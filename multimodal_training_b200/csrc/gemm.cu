@@ -222,7 +222,7 @@ struct Cfg {
   static constexpr int kStages = (int)((227u * 1024u - 2048u - STORE_BYTES) / STAGE_BYTES) > 8
                                      ? 8 : (int)((227u * 1024u - 2048u - STORE_BYTES) / STAGE_BYTES);
   static constexpr uint32_t TMEM_COLS = (2 * BN <= 128) ? 128 : (2 * BN <= 256 ? 256 : 512);
-  static constexpr size_t SMEM = 1024 + (size_t)kStages * STAGE_BYTES + STORE_BYTES + (4 * kStages + 4) * 8 + 16;
+  static constexpr size_t SMEM = 1024 + (size_t)kStages * STAGE_BYTES + STORE_BYTES + (4 * kStages + 5) * 8 + 16;
   static_assert(MT == 1 || 2 * BN <= 512, "two accumulators must fit tensor memory");
 };
 
@@ -691,8 +691,6 @@ MMT_DEVICE void epilogue_partial(uint32_t tmem_acc, float* dst, int q, int half,
   }
 }
 
-MMT_DEVICE void epi_bar_sync() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
-
 // Does the CTA that computes tile (tm, tn) also forward the tile's rows of A to the peers?  (GemmParams::fwd_peers)
 MMT_DEVICE bool forwards_tile(const GemmParams& p, int tm, int tn, int bmt) {
   if (p.fwd_peers <= 0 || tn >= p.fwd_split) return false;
@@ -741,7 +739,8 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   // one phase per FORWARDED use of a stage, and each has a single waiter that follows every phase.
   uint64_t* fwd_go = tempty + 2;          // [kStages]
   uint64_t* fwd_done = fwd_go + kStages;  // [kStages]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fwd_done + kStages);
+  uint64_t* sk_stored = fwd_done + kStages;   // stream-K: every epilogue warp has stored its part of the partial sums
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sk_stored + 1);
 
   const int warp = warp_uniform((int)threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -765,6 +764,7 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     mbar_init(&tfull[1], 1);
     mbar_init(&tempty[0], kEpiWarps);
     mbar_init(&tempty[1], kEpiWarps);
+    mbar_init(sk_stored, kEpiWarps);
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -1065,10 +1065,17 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
       if (!ok) break;
       if (w.kind == 1) {
-        // every epilogue warp has stored its part: publish "the partial sums of CTA blockIdx.x are complete"
+        // every epilogue warp has stored its part: publish "the partial sums of CTA blockIdx.x are complete".  (A run has
+        // at most one such item, so the barrier is used once.  It is one with a limit: a warp whose accumulator never
+        // came has left the loop above.)
         __threadfence();
-        epi_bar_sync();
-        if (warp == 2 && lane == 0) flag_store_release_sys(&p.sk_flags[blockIdx.x], p.sk_epoch);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sk_stored);
+        if (warp == 2) {
+          ok = mbar_wait_warp(sk_stored, 0, p.ew, 311);
+          if (!ok) break;
+          if (lane == 0) flag_store_release_sys(&p.sk_flags[blockIdx.x], p.sk_epoch);
+        }
       }
       if (MT == 1) {
         acc ^= 1;
