@@ -1398,16 +1398,18 @@ int g_sk_epoch = 0;
 // training step at the board's power cap its extra partial-sum traffic costs as much as the idle SMs it fills
 // (7B step on one B200: 204.5 ms without, 205.9 ms with).
 int g_sk_mode = -1;           // 1 = on, 0 = off, -1 = not yet read from the environment
-double g_mt2_const = -1.0;    // fixed cost of a 256-row tile in the tile-shape model (MMT_GEMM_MT2_CONST overrides)
+double g_mt2_const = -1.0;    // fixed cost of a 256-row tile in the tile-shape models (MMT_GEMM_MT2_CONST), < 0: theirs
+bool g_env_read = false;
 
 void read_env_once() {
   if (g_sk_mode < 0) {
     const char* e = getenv("MMT_GEMM_STREAM_K");
     g_sk_mode = (e && e[0] == '1') ? 1 : 0;
   }
-  if (g_mt2_const < 0.0) {
+  if (!g_env_read) {
     const char* e = getenv("MMT_GEMM_MT2_CONST");
-    g_mt2_const = e ? atof(e) : 3.8;
+    if (e) g_mt2_const = atof(e);
+    g_env_read = true;
   }
 }
 cudaEvent_t g_sk_event = nullptr;
@@ -1638,12 +1640,12 @@ struct GemmCount {
   int mt, bn;
 };
 
-// Model of the persistent kernel's time, see gemm_call.
+// Model of the persistent kernel's time for a product without collective roles, in us, see choose_tile.
 static double wave_cost(int M, int N, long kb, int sms, int m, int width, bool stream_k) {
   const long tiles = (long)((M + 128 * m - 1) / (128 * m)) * ((N + width - 1) / width);
   const long full = tiles / sms, rem = tiles % sms;
   double c, e;
-  if (width == 256) { c = m == 2 ? 0.636 : 0.39; e = m == 2 ? g_mt2_const : 0.5; }
+  if (width == 256) { c = m == 2 ? 0.636 : 0.39; e = m == 2 ? (g_mt2_const >= 0.0 ? g_mt2_const : 3.8) : 0.5; }
   else              { c = m == 2 ? 0.56 : 0.33; e = m == 2 ? 2.2 : 0.6; }
   if (rem && stream_k && width == 256 && sk_tiles_for((int)tiles, kb, sms, m) > 0)
     return ((double)full + (double)rem / sms + (m == 2 ? 16.0 : 8.0) / (double)kb) * ((double)kb * c + e);
@@ -1651,38 +1653,41 @@ static double wave_cost(int M, int N, long kb, int sms, int m, int width, bool s
   return full * ((double)kb * c + e) + last;
 }
 
-static int gemm_call(const void* A, const void* B, void* C, const void* bias, const void* residual, int M, int N, int K,
-                     int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int act, int accumulate, int out_f32,
-                     float alpha, int bn, const GemmCount* count, void* stream) {
-  // collective roles belong to THIS call only: take them before any early return, so that a call that fails its
-  // argument checks cannot leave them behind for an unrelated GEMM
-  const MmtGemmComm* comm = g_comm;
-  g_comm = nullptr;
-  if (M <= 0 || N <= 0 || K <= 0) return comm ? -9 : 0;     // peers would wait for flags that an empty GEMM never sets
-  if (mmt_ensure_context(A)) return -7;
-  if ((lda & 7) || (ldb & 7) || (ldc & 7) || (N & 7) || (residual && (ldr & 7))) return -2;
-  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
-      (reinterpret_cast<uintptr_t>(C) & 15))
-    return -3;
-  const int sms = mmt_sm_count();
-  // Tile shape: rows = 128 (accumulator double buffered in tensor memory, epilogue hidden behind the next tile) or
-  // 256 (two accumulators that share every B tile: the main loop alternates between them, which keeps the tensor pipe
-  // busier than back-to-back MMAs into one accumulator, but the two fill tensor memory and the epilogue is exposed);
-  // width = 192 or 256 columns (narrower only for narrow outputs: a 128-wide MMA is bound by shared-memory reads).
-  // Cost of a candidate in us = waves x (k-blocks x c + e), with c and e from single GEMMs of 1600 to 16384 rows and K of
-  // 1280 to 6848 in a graph (rows x width: 128 x 256 c 0.39 e 0.5; 256 x 256 c 0.636 e 3.8; 128 x 192 c 0.33 e 0.6;
-  // 256 x 192 c 0.56 e 2.2).  c is close to what one SM's operand intake (about 110 GB/s) allows, so wide tiles win for
-  // long K; e is the exposed epilogue of a 256-row tile, so 128-row tiles win for short K.  A last wave that is partly
-  // empty has the L2 to itself and is up to a fifth faster.  What it mostly decides is how well the tile count fills
-  // the 148 SMs.  (Constants from the time when issuing paced the 128-row tiles preferred 256 rows more often: 16384 x
-  // 1280 x 1280 62.5 -> 50.6 us, 16384 x 1280 x 3840 135 -> 125, 6000 x 3840 x 1280 53.7 -> 49.1.)
-  read_env_once();
+// The same for a product with collective roles, in units of one 256 x 256 x 64 step: waves x (k-blocks x c + e), with c and
+// e fitted (least squares over 200 sustained measurements on B200: the text shapes, the short-K vision shapes and the
+// tensor-parallel shards, all layouts).  Operand tiles that other ranks deliver are still fetched by a producer that one
+// lane runs, which is what these constants were taken with and those above were not.
+static double collective_cost(int M, int N, long kb, int sms, int m, int width) {
+  const long tiles = (long)((M + 128 * m - 1) / (128 * m)) * ((N + width - 1) / width);
+  const double waves = (double)((tiles + sms - 1) / sms);
+  double c, e;
+  if (width == 256) { c = m == 2 ? 0.824 : 0.568; e = m == 2 ? (g_mt2_const >= 0.0 ? g_mt2_const : 4.06) : 0.86; }
+  else              { c = m == 2 ? 0.726 : 0.507; e = m == 2 ? 2.61 : 0.4; }
+  return waves * ((double)kb * c + e);
+}
+
+struct Tile {
+  int mt, bn;               // 128-row accumulators, columns
+};
+
+// Tile shape: rows = 128 (accumulator double buffered in tensor memory, epilogue hidden behind the next tile) or
+// 256 (two accumulators that share every B tile: the main loop alternates between them, which keeps the tensor pipe
+// busier than back-to-back MMAs into one accumulator, but the two fill tensor memory and the epilogue is exposed);
+// width = 192 or 256 columns (narrower only for narrow outputs: a 128-wide MMA is bound by shared-memory reads).
+// Cost of a candidate in us = waves x (k-blocks x c + e), with c and e from single GEMMs of 1600 to 16384 rows and K of
+// 1280 to 6848 in a graph (rows x width: 128 x 256 c 0.39 e 0.5; 256 x 256 c 0.636 e 3.8; 128 x 192 c 0.33 e 0.6;
+// 256 x 192 c 0.56 e 2.2).  c is close to what one SM's operand intake (about 110 GB/s) allows, so wide tiles win for
+// long K; e is the exposed epilogue of a 256-row tile, so 128-row tiles win for short K.  A last wave that is partly
+// empty has the L2 to itself and is up to a fifth faster.  What it mostly decides is how well the tile count fills
+// the 148 SMs.  (Constants from the time when issuing paced the 128-row tiles preferred 256 rows more often: 16384 x
+// 1280 x 1280 62.5 -> 50.6 us, 16384 x 1280 x 3840 135 -> 125, 6000 x 3840 x 1280 53.7 -> 49.1.)
+// Products with collective roles keep those earlier constants, see collective_cost.
+// bn: 0 = choose, else the width asked for.
+static Tile choose_tile(int M, int N, long kb, int sms, int bn, bool collective) {
+  auto cost = [&](int m, int width) {
+    return collective ? collective_cost(M, N, kb, sms, m, width) : wave_cost(M, N, kb, sms, m, width, true);
+  };
   int mt = 1;
-  const long kb = (K + BK - 1) / BK;
-  const bool plain = comm == nullptr;
-  auto cost = [&](int m, int width) { return wave_cost(M, N, kb, sms, m, width, plain); };
-  if (bn == 0 && g_force_bn) bn = g_force_bn;
-  const bool choose = bn == 0 && g_force_mt == 0 && !g_use_pair && !count;
   if (bn == 0 && N <= 192) bn = N > 128 ? 192 : (N > 64 ? 128 : 64);
   if (bn == 0) {
     double best = 1e30;
@@ -1701,6 +1706,38 @@ static int gemm_call(const void* A, const void* B, void* C, const void* bias, co
   } else if (g_force_mt == 2 && M >= 256 && bn == 128) {
     mt = 2;
   }
+  return {mt, bn};
+}
+
+// The choice for a product on `sms` SMs: 128-row accumulators x 1000 + columns (tests).
+extern "C" int mmt_gemm_tile_choice(int M, int N, int K, int sms, int collective) {
+  read_env_once();
+  const Tile t = choose_tile(M, N, (K + BK - 1) / BK, sms, 0, collective != 0);
+  return t.mt * 1000 + t.bn;
+}
+
+static int gemm_call(const void* A, const void* B, void* C, const void* bias, const void* residual, int M, int N, int K,
+                     int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int act, int accumulate, int out_f32,
+                     float alpha, int bn, const GemmCount* count, void* stream) {
+  // collective roles belong to THIS call only: take them before any early return, so that a call that fails its
+  // argument checks cannot leave them behind for an unrelated GEMM
+  const MmtGemmComm* comm = g_comm;
+  g_comm = nullptr;
+  if (M <= 0 || N <= 0 || K <= 0) return comm ? -9 : 0;     // peers would wait for flags that an empty GEMM never sets
+  if (mmt_ensure_context(A)) return -7;
+  if ((lda & 7) || (ldb & 7) || (ldc & 7) || (N & 7) || (residual && (ldr & 7))) return -2;
+  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
+      (reinterpret_cast<uintptr_t>(C) & 15))
+    return -3;
+  const int sms = mmt_sm_count();
+  read_env_once();
+  const long kb = (K + BK - 1) / BK;
+  const bool plain = comm == nullptr;
+  if (bn == 0 && g_force_bn) bn = g_force_bn;
+  const bool choose = bn == 0 && g_force_mt == 0 && !g_use_pair && !count;
+  const Tile tile = choose_tile(M, N, kb, sms, bn, !plain);
+  int mt = tile.mt;
+  bn = tile.bn;
   if (bn == 256 && M >= 256 && (g_force_mt == 3 || (g_use_pair && g_force_mt == 0)) && !(comm && (comm->fwd_peers > 0 || comm->sc_row || comm->kf_flags)))
     mt = 3;   // 2-CTA kernel
   if (count && count->mt) {
