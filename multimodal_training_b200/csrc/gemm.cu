@@ -1947,16 +1947,21 @@ extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* 
 // or over that many of the K rows of MN-major A and B (is_k == 1; see GemmParams::cnt for the zeros it needs).  The host
 // does not know the count, and which tile is best depends on it: a row count is cut into up to 32 buckets, and every
 // tile that is the best of some bucket is launched; the launches that the count does not belong to return at once.
+// *launches: how many kernels this call has launched.
 extern "C" int mmt_gemm_bf16_counted(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                                     int a_mn, int b_mn, int accumulate, const int* cnt, int is_k, void* stream) {
+                                     int a_mn, int b_mn, int accumulate, const int* cnt, int is_k, int* launches,
+                                     void* stream) {
+  *launches = 0;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   GemmCount c = {cnt, is_k, 1, 0u, 0, 0};
+  *launches = 1;
   if (is_k)
     return gemm_call(A, B, C, nullptr, nullptr, M, N, K, lda, ldb, ldc, 0, a_mn, b_mn, 0, accumulate, 0, 1.f, 0, &c, stream);
   read_env_once();
   const int sms = mmt_sm_count();
   const long kb = (K + BK - 1) / BK;
   c.bucket = ((M + 31) / 32 + 127) / 128 * 128;
+  *launches = 0;
   uint32_t mask[4] = {0, 0, 0, 0};                       // 128 x 192, 128 x 256, 256 x 192, 256 x 256
   for (int b = 0; b * c.bucket < M; ++b) {
     int best = 0;
@@ -1974,6 +1979,7 @@ extern "C" int mmt_gemm_bf16_counted(const void* A, const void* B, void* C, int 
     const int rc = gemm_call(A, B, C, nullptr, nullptr, M, N, K, lda, ldb, ldc, 0, a_mn, b_mn, 0, accumulate, 0, 1.f, c.bn,
                              &c, stream);
     if (rc) return rc;
+    ++*launches;
   }
   return 0;
 }

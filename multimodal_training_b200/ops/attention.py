@@ -152,6 +152,8 @@ def attn_bwd(qkv, out, dout, lse, n_q: int, n_kv: int, dim: int, info: SeqInfo, 
     nv.call("mmt_attn_bwd", qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), delta.data_ptr(),
             dqkv.data_ptr(), lo.data_ptr(), hi.data_ptr(), T, n_q, n_kv, dim, qkv.stride(0), int(causal), scale,
             nv.ptr(ws), nv.stream())
+    if ws is not None:
+        nv.launch_count += 1                       # the sum over a group's heads
     return dqkv
 
 

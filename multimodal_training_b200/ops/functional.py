@@ -15,6 +15,7 @@ add pass.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
@@ -88,8 +89,11 @@ def _gemm_counted(a, b, out, count: torch.Tensor, *, of_k: bool = False, a_mn: b
     assert K == (b.shape[0] if b_mn else b.shape[1]) and out.shape == (M, N)
     if M == 0 or K == 0:
         return
+    launches = ctypes.c_int()
     nv.call("mmt_gemm_bf16_counted", a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-            out.stride(0), int(a_mn), int(b_mn), int(accumulate), count.data_ptr(), int(of_k), nv.stream())
+            out.stride(0), int(a_mn), int(b_mn), int(accumulate), count.data_ptr(), int(of_k), ctypes.byref(launches),
+            nv.stream())
+    nv.launch_count += launches.value - 1          # nv.call has counted one
 
 
 def _write_param_grad(p: torch.Tensor, compute) -> torch.Tensor | None:

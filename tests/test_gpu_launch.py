@@ -50,3 +50,32 @@ def test_back_to_back_equals_one_at_a_time(rows, monkeypatch):
     for got in queued + [captured]:
         assert torch.equal(got, want)
     assert nv.get_error()[0] == 0
+
+
+def test_launch_count_is_what_ran():
+    """Calls that launch a number of kernels which depends on their sizes."""
+    from multimodal_training_b200.ops import functional as F
+    from multimodal_training_b200.ops import native as nv
+    from multimodal_training_b200.ops.attention import SeqInfo
+    g = torch.Generator().manual_seed(3)
+    h = torch.randn(1500, 256, generator=g).cuda().bfloat16().requires_grad_()
+    w = (torch.randn(38016, 256, generator=g) * 0.1).cuda().bfloat16().requires_grad_()
+    labels = torch.randint(0, 38016, (1500,), generator=g).cuda()
+    seq = SeqInfo.from_list([0, 300], "cuda")
+    qkv = {n_kv: torch.randn(300, (4 + 2 * n_kv) * 128, generator=g).cuda().bfloat16().requires_grad_() for n_kv in (2, 4)}
+
+    def work():
+        F.lm_head_cross_entropy(h, w, labels, chunk_rows=700).backward()
+        for n_kv, t in qkv.items():
+            F.attention(t, 4, n_kv, 128, seq, causal=True).sum().backward()
+
+    work()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        before = nv.launch_count
+        work()
+        torch.cuda.synchronize()
+        counted = nv.launch_count - before
+    names = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    own = [n for n in names if not any(s in n for s in ("at::", "cub::", "Memset", "Memcpy"))]
+    assert counted == len(own), (counted, sorted(own))
