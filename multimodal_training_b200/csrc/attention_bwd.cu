@@ -20,7 +20,7 @@ using namespace attn;
 // ----------------------------------------------------------------------------------------------
 // 1. delta
 // ----------------------------------------------------------------------------------------------
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
+__global__ void attn_delta_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout,
                                   float* __restrict__ delta, int T, int n_q, int dim) {
   grid_dependency_sync();
   const long w = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
@@ -41,7 +41,7 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const _
 }
 
 // dK / dV of a GQA group = sum of its q heads' fp32 partials, in head order (deterministic), rounded once.
-__global__ void attn_group_reduce_kernel(const float* __restrict__ ws_dk, const float* __restrict__ ws_dv,
+__global__ void attn_group_reduce_kernel(const float* ws_dk, const float* ws_dv,
                                          __nv_bfloat16* __restrict__ dqkv, int T, int n_q, int n_kv, int dim, long ld) {
   grid_dependency_sync();
   const int group = n_q / n_kv;

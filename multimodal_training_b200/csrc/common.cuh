@@ -64,6 +64,11 @@ MMT_DEVICE uint64_t mmt_globaltimer() {
 // this grid leaves free.  Nothing in front of it may touch global memory (barrier set-up, tensor-memory allocation and
 // descriptor prefetches may); EVERY thread block has to execute it, so that "this grid has finished" implies the same
 // of all grids before it.
+// What such a kernel reads may be written while it already runs, in front of that statement.  So it reads through ordinary
+// loads: a pointer parameter that is `const` and `__restrict__` (or __ldg) promises data that does not change during the
+// kernel, for which the compiler may use the read-only path, whose lines nothing refreshes, and which it may move up.  The
+// same goes for __restrict__ on a buffer that is read and written in place.  Outputs that are only written keep it, which
+// is what lets loads pass their stores.
 MMT_DEVICE void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 MMT_DEVICE void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 MMT_DEVICE void grid_dependency_sync() {

@@ -79,8 +79,8 @@ MMT_DEVICE float block_max(float v, float* red) {
 constexpr int kNormThreads = 256;
 constexpr int kNormVec = 4;  // up to 8192 columns
 
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_fwd_kernel(const bf16* __restrict__ x,
-                                                                  const bf16* __restrict__ w, bf16* __restrict__ y,
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_fwd_kernel(const bf16* x,
+                                                                  const bf16* w, bf16* __restrict__ y,
                                                                   float* __restrict__ rstd_out, int cols, float eps) {
   grid_dependency_sync();
   __shared__ float red[32];
@@ -127,8 +127,8 @@ MMT_DEVICE void unpack8(const uint4& u, float (&v)[8]) {
 // Forward for rows of up to 4096 columns: one warp per row (the row stays in registers as raw bf16, the sum of
 // squares needs shuffles only), eight rows per CTA, no block-wide barrier.
 template <int VPL>
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_fwd_warp_kernel(const bf16* __restrict__ x,
-                                                                       const bf16* __restrict__ w,
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_fwd_warp_kernel(const bf16* x,
+                                                                       const bf16* w,
                                                                        bf16* __restrict__ y,
                                                                        float* __restrict__ rstd_out, long rows,
                                                                        int cols, float eps) {
@@ -177,13 +177,13 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_fwd_warp_kernel(const bf
 // dots (one __syncthreads per iteration, the exchange buffer alternates), which keeps enough bytes in flight per SM
 // to run at memory speed; the rows are held as raw bf16 so that R x VEC vectors fit in registers.
 template <int VEC, int R>
-__global__ void __launch_bounds__(kNormThreads, VEC <= 2 ? 2 : 1) rmsnorm_bwd_kernel(const bf16* __restrict__ dy,
-                                                                     const bf16* __restrict__ x,
-                                                                     const bf16* __restrict__ w,
-                                                                     const float* __restrict__ rstd_in,
+__global__ void __launch_bounds__(kNormThreads, VEC <= 2 ? 2 : 1) rmsnorm_bwd_kernel(const bf16* dy,
+                                                                     const bf16* x,
+                                                                     const bf16* w,
+                                                                     const float* rstd_in,
                                                                      bf16* __restrict__ dx,
                                                                      float* __restrict__ dw_partial, int rows, int cols,
-                                                                     const bf16* __restrict__ extra) {
+                                                                     const bf16* extra) {
   grid_dependency_sync();
   constexpr int kWarps = kNormThreads / 32;
   __shared__ float red[2][R][kWarps];
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const ReduceSegmen
 // x: [tokens, row_stride] with head h at column h*dim; cs: cos [tokens, dim], sin [tokens, dim] (fp32).
 // sign = +1 forward, -1 backward (the transpose of the rotation).
 // ----------------------------------------------------------------------------
-__global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+__global__ void rope_kernel(bf16* x, const float* cos_t, const float* sin_t,
                             long tokens, int heads, int dim, long row_stride, float sign) {
   grid_dependency_sync();
   const int half = dim >> 1;
@@ -355,9 +355,9 @@ __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cos_
 // entries are four times the bytes of the data they rotate; read once per HPT heads they no longer fill the load path.
 // Measured, 32 heads of 80: 4096 tokens 11.6 -> 10.0 us, 16384 tokens 36.6 -> 31.8 us (the bytes alone: 6.4 and 26 us).
 template <int HPT>
-__global__ void __launch_bounds__(256, HPT == 1 ? 4 : 2) rope_vec8_kernel(bf16* __restrict__ x,
-                                                                         const float* __restrict__ cos_t,
-                                                                         const float* __restrict__ sin_t, long tokens,
+__global__ void __launch_bounds__(256, HPT == 1 ? 4 : 2) rope_vec8_kernel(bf16* x,
+                                                                         const float* cos_t,
+                                                                         const float* sin_t, long tokens,
                                                                          int heads, int dim, long row_stride, float sign) {
   grid_dependency_sync();
   const int half = dim >> 1;
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(256, HPT == 1 ? 4 : 2) rope_vec8_kernel(bf16* 
 // ----------------------------------------------------------------------------
 // SwiGLU on a fused [rows, 2*inter] gate|up buffer.
 // ----------------------------------------------------------------------------
-__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long rows, int inter) {
+__global__ void swiglu_fwd_kernel(const bf16* gu, bf16* __restrict__ out, long rows, int inter) {
   grid_dependency_sync();
   const int nvec = inter >> 3;
   const long total = rows * nvec;
@@ -430,7 +430,7 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
   }
 }
 
-__global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu,
+__global__ void swiglu_bwd_kernel(const bf16* dout, const bf16* gu, bf16* __restrict__ dgu,
                                   long rows, int inter) {
   grid_dependency_sync();
   const int nvec = inter >> 3;
@@ -454,7 +454,7 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __r
   }
 }
 
-__global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long n8) {
+__global__ void gelu_fwd_kernel(const bf16* x, bf16* __restrict__ y, long n8) {
   grid_dependency_sync();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
     float v[8];
@@ -464,7 +464,7 @@ __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y
     store8(y + i * 8, v);
   }
 }
-__global__ void gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, bf16* __restrict__ dx,
+__global__ void gelu_bwd_kernel(const bf16* dy, const bf16* x, bf16* __restrict__ dx,
                                 long n8) {
   grid_dependency_sync();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
@@ -478,7 +478,7 @@ __global__ void gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restr
 }
 
 // y = a + b (bf16), used for residual adds outside GEMM epilogues.
-__global__ void add_kernel(const bf16* __restrict__ a, const bf16* __restrict__ b, bf16* __restrict__ y, long n8) {
+__global__ void add_kernel(const bf16* a, const bf16* b, bf16* __restrict__ y, long n8) {
   grid_dependency_sync();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
     float u[8], v[8];
@@ -494,7 +494,7 @@ __global__ void add_kernel(const bf16* __restrict__ a, const bf16* __restrict__ 
 // Row gather / scatter.  idx[r] < 0 (or outside [lo, hi)) gives a zero row on
 // gather and is skipped on scatter.  One warp per row.
 // ----------------------------------------------------------------------------
-__global__ void gather_rows_kernel(const bf16* __restrict__ src, const long* __restrict__ idx, bf16* __restrict__ dst,
+__global__ void gather_rows_kernel(const bf16* src, const long* idx, bf16* __restrict__ dst,
                                    long rows, int cols, long lo, long hi, long src_ld, long dst_ld) {
   grid_dependency_sync();
   const long r = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -502,15 +502,22 @@ __global__ void gather_rows_kernel(const bf16* __restrict__ src, const long* __r
   const int lane = threadIdx.x & 31;
   const long s = idx[r];
   const bool valid = s >= lo && s < hi;
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  for (int c = lane * 8; c < cols; c += 256) {
-    uint4 v = valid ? *reinterpret_cast<const uint4*>(src + (s - lo) * src_ld + c) : zero;
-    *reinterpret_cast<uint4*>(dst + r * dst_ld + c) = v;
+  // four loads in flight before the first store
+  for (int c0 = lane * 8; c0 < cols; c0 += 4 * 256) {
+    uint4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = make_uint4(0, 0, 0, 0);
+      if (valid && c0 + k * 256 < cols) v[k] = *reinterpret_cast<const uint4*>(src + (s - lo) * src_ld + c0 + k * 256);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (c0 + k * 256 < cols) *reinterpret_cast<uint4*>(dst + r * dst_ld + c0 + k * 256) = v[k];
   }
 }
 
 // dst[idx[r]] = src[r]   (add == 0)   or   dst[idx[r]] += src[r]  (add == 1, bf16x2 atomics)
-__global__ void scatter_rows_kernel(const bf16* __restrict__ src, const long* __restrict__ idx, bf16* __restrict__ dst,
+__global__ void scatter_rows_kernel(const bf16* src, const long* idx, bf16* dst,
                                     long rows, int cols, long lo, long hi, long src_ld, long dst_ld, int add) {
   grid_dependency_sync();
   const long r = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -519,12 +526,24 @@ __global__ void scatter_rows_kernel(const bf16* __restrict__ src, const long* __
   const long d = idx[r];
   if (d < lo || d >= hi) return;
   if (!add) {
-    for (int c = lane * 8; c < cols; c += 256)
-      *reinterpret_cast<uint4*>(dst + (d - lo) * dst_ld + c) = *reinterpret_cast<const uint4*>(src + r * src_ld + c);
+    for (int c0 = lane * 8; c0 < cols; c0 += 4 * 256) {
+      uint4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c0 + k * 256 < cols) v[k] = *reinterpret_cast<const uint4*>(src + r * src_ld + c0 + k * 256);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c0 + k * 256 < cols) *reinterpret_cast<uint4*>(dst + (d - lo) * dst_ld + c0 + k * 256) = v[k];
+    }
   } else {
-    for (int c = lane * 2; c < cols; c += 64) {
-      const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(src + r * src_ld + c);
-      atomicAdd(reinterpret_cast<__nv_bfloat162*>(dst + (d - lo) * dst_ld + c), v);
+    for (int c0 = lane * 2; c0 < cols; c0 += 4 * 64) {
+      __nv_bfloat162 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c0 + k * 64 < cols) v[k] = *reinterpret_cast<const __nv_bfloat162*>(src + r * src_ld + c0 + k * 64);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c0 + k * 64 < cols) atomicAdd(reinterpret_cast<__nv_bfloat162*>(dst + (d - lo) * dst_ld + c0 + k * 64), v[k]);
     }
   }
 }
@@ -532,7 +551,7 @@ __global__ void scatter_rows_kernel(const bf16* __restrict__ src, const long* __
 // ----------------------------------------------------------------------------
 // Column sums: out[c] (+)= sum_r x[r, c].  Stage 1 writes per-CTA partials.
 // ----------------------------------------------------------------------------
-__global__ void colsum_partial_kernel(const bf16* __restrict__ x, float* __restrict__ partial, long rows, int cols,
+__global__ void colsum_partial_kernel(const bf16* x, float* __restrict__ partial, long rows, int cols,
                                       long ld) {
   grid_dependency_sync();
   // blockDim = (32 column-vectors, 8 row lanes); grid = (ceil(cols/256), row splits)
@@ -570,10 +589,10 @@ __global__ void colsum_partial_kernel(const bf16* __restrict__ x, float* __restr
 // ----------------------------------------------------------------------------
 constexpr int kCeThreads = 512;
 
-__global__ void __launch_bounds__(kCeThreads) ce_stats_kernel(const bf16* __restrict__ logits,
-                                                             const long* __restrict__ labels, float* __restrict__ omax,
+__global__ void __launch_bounds__(kCeThreads) ce_stats_kernel(const bf16* logits,
+                                                             const long* labels, float* __restrict__ omax,
                                                              float* __restrict__ osum, float* __restrict__ otgt, int V,
-                                                             long ld, long vocab_lo, const long* __restrict__ pos,
+                                                             long ld, long vocab_lo, const long* pos,
                                                              long base) {
   grid_dependency_sync();
   __shared__ float red[32];
@@ -613,12 +632,12 @@ __global__ void __launch_bounds__(kCeThreads) ce_stats_kernel(const bf16* __rest
   }
 }
 
-__global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* __restrict__ logits, const long* __restrict__ labels,
-                                                            const float* __restrict__ gmax,
-                                                            const float* __restrict__ gsum,
-                                                            const float* __restrict__ scale_ptr, int V, long ld,
-                                                            long vocab_lo, const int* __restrict__ cnt,
-                                                            const long* __restrict__ src, long base) {
+__global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* logits, const long* labels,
+                                                            const float* gmax,
+                                                            const float* gsum,
+                                                            const float* scale_ptr, int V, long ld,
+                                                            long vocab_lo, const int* cnt,
+                                                            const long* src, long base) {
   grid_dependency_sync();
   const long row = blockIdx.x;
   bf16* l = logits + row * ld;
@@ -665,7 +684,7 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_kernel(bf16* __restrict__ 
 // ----------------------------------------------------------------------------
 constexpr int kCompactThreads = 1024;
 constexpr int kLabelBlock = 64;
-__global__ void __launch_bounds__(kCompactThreads) compact_labels_kernel(const long* __restrict__ labels, long n, long chunk,
+__global__ void __launch_bounds__(kCompactThreads) compact_labels_kernel(const long* labels, long n, long chunk,
                                                                         long* __restrict__ src, long* __restrict__ lab,
                                                                         long* __restrict__ pos, int* __restrict__ count) {
   grid_dependency_sync();
@@ -712,10 +731,10 @@ __global__ void __launch_bounds__(kCompactThreads) compact_labels_kernel(const l
 //   g <- g * gscale;  m,v update;  master -= lr * (mhat / (sqrt(vhat) + eps) + wd * master);  p = bf16(master)
 // Elements [0, n_decay) use `wd`, the rest 0.  gscale_ptr may be null (1.0).
 // ----------------------------------------------------------------------------
-__global__ void adamw_kernel(bf16* __restrict__ p, const bf16* __restrict__ g, float* __restrict__ master,
-                             float* __restrict__ m, float* __restrict__ v, long n, long n_decay, float lr, float b1,
+__global__ void adamw_kernel(bf16* __restrict__ p, const bf16* g, float* master,
+                             float* m, float* v, long n, long n_decay, float lr, float b1,
                              float b2, float eps, float wd, float bc1, float bc2,
-                             const float* __restrict__ gscale_ptr) {
+                             const float* gscale_ptr) {
   grid_dependency_sync();
   const float gs = gscale_ptr ? *gscale_ptr : 1.f;
   const long n8 = n >> 3;
@@ -753,9 +772,9 @@ __global__ void adamw_kernel(bf16* __restrict__ p, const bf16* __restrict__ g, f
 // bf16 model, the reference's setting: python/ray/trainer.py:503-572): no fp32 master copy, moments in bf16.  The
 // arithmetic of an element is fp32; weight, m and v are rounded to bf16 when stored.  14 bytes of traffic per
 // parameter instead of 28.
-__global__ void adamw_bf16_kernel(bf16* __restrict__ p, const bf16* __restrict__ g, bf16* __restrict__ m,
-                                  bf16* __restrict__ v, long n, long n_decay, float lr, float b1, float b2, float eps,
-                                  float wd, float bc1, float bc2, const float* __restrict__ gscale_ptr) {
+__global__ void adamw_bf16_kernel(bf16* p, const bf16* g, bf16* m,
+                                  bf16* v, long n, long n_decay, float lr, float b1, float b2, float eps,
+                                  float wd, float bc1, float bc2, const float* gscale_ptr) {
   grid_dependency_sync();
   const float gs = gscale_ptr ? *gscale_ptr : 1.f;
   const long n8 = n >> 3;
@@ -782,7 +801,7 @@ __global__ void adamw_bf16_kernel(bf16* __restrict__ p, const bf16* __restrict__
 }
 
 // out[0] += sum(x^2)   (fp32 atomic; caller zeroes out)
-__global__ void sumsq_kernel(const bf16* __restrict__ x, long n8, float* __restrict__ out) {
+__global__ void sumsq_kernel(const bf16* x, long n8, float* out) {
   grid_dependency_sync();
   __shared__ float red[32];
   float s = 0.f;
@@ -797,7 +816,7 @@ __global__ void sumsq_kernel(const bf16* __restrict__ x, long n8, float* __restr
 }
 
 // coef = min(1, max_norm / (sqrt(normsq) + 1e-6)) * extra
-__global__ void clip_coef_kernel(const float* __restrict__ normsq, float max_norm, float extra,
+__global__ void clip_coef_kernel(const float* normsq, float max_norm, float extra,
                                  float* __restrict__ coef) {
   grid_dependency_sync();
   const float n = sqrtf(*normsq);

@@ -539,7 +539,7 @@ MMT_DEVICE void epilogue_fast(const GemmParams& p, const OutMaps& tmC, uint32_t 
       if (kBias || kResid) {
         if (col < N) {
           if (kBias) {
-            const uint4 bv = __ldg(reinterpret_cast<const uint4*>(p.bias + col));
+            const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
             const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
