@@ -450,8 +450,8 @@ class _LMHeadCEFn(torch.autograd.Function):
             else:
                 dw = mg
                 acc0 = bool(getattr(weight, "grad_written", False))
-        # Rows without a label (image tokens, prompts, the last token of a sample) have no loss and no gradient: blocks of
-        # rows that have none are left out, the others of a chunk move to its front, and the products below stop behind
+        # Rows without a label (image tokens, prompts, the last token of a sample) have no loss and no gradient: groups of
+        # 16 rows that have none are left out, the others of a chunk move to its front, and the products below stop behind
         # the last of them.  Their number stays on the device.  (Label smoothing works on plain tensors of all rows.)
         # Half of a sample's rows are image tokens in the 7B configuration, two thirds in the 32B one.
         x, labs, dx, count, src, pos = hidden, labels, dhidden, None, None, None
