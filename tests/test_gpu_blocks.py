@@ -72,3 +72,77 @@ def test_gradient_views_with_gaps(kind, written):
         got.append({n: t.main_grad for n, t in p.items() if t is not None})
     for n, g in got[0].items():
         assert torch.equal(g, got[1][n]), n
+
+
+# the last sequence crosses a tile (general attention kernels) or none does (the kernels for short sequences; with grouped
+# heads their forward and the general backward)
+SEQS = [[0, 64, 128, 192, 300], [0, 64, 128, 192, 256, 300], [0, 100, 128, 200], [0, 200, 456]]
+
+
+def _per_op(kind, x, cos, sin, seq, p):
+    from multimodal_training_b200.ops import functional as F
+    n_q, n_kv, d, _, _, causal, _ = _shape(kind)
+    h = F.rmsnorm(x, p["ln1"], 1e-6)
+    qkv = F.rope(F.linear(h, p["qkv_w"], p["qkv_b"]), cos, sin, n_q + n_kv, d)
+    x1 = F.linear(F.attention(qkv, n_q, n_kv, d, seq, causal=causal), p["o_w"], p["o_b"], x)
+    m = F.swiglu(F.linear(F.rmsnorm(x1, p["ln2"], 1e-6), p["gu_w"], p["gu_b"]))
+    return F.linear(m, p["dn_w"], p["dn_b"], x1)
+
+
+@pytest.mark.parametrize("cu", SEQS)
+@pytest.mark.parametrize("kind", ["vision", "text"])
+def test_without_gradients_the_bits_of_the_per_op_graph(kind, cu):
+    from multimodal_training_b200.ops.attention import SeqInfo
+    x, _, cos, sin = _inputs(kind, cu[-1])
+    p = _params(kind)
+    with torch.no_grad():
+        want = _per_op(kind, x, cos, sin, SeqInfo.from_list(cu, DEV), p)
+        for seq in (SeqInfo.from_list(cu, DEV), cu):
+            assert torch.equal(_block(kind, x, cos, sin, seq, p, 2), want)
+
+
+@pytest.mark.parametrize("written", [False, True])
+@pytest.mark.parametrize("cu", SEQS)
+@pytest.mark.parametrize("kind", ["vision", "text"])
+def test_gradients_in_views(kind, cu, written):
+    """Into the views of a flat buffer, over what is there or added to it: the same bits whatever is kept for backward,
+    and the per-op graph's values up to the rounding of the residual sums."""
+    from multimodal_training_b200.ops import native as nv
+    from multimodal_training_b200.ops.attention import SeqInfo
+    x, dy, cos, sin = _inputs(kind, cu[-1])
+    got = []
+    for run in (lambda *a: _per_op(*a), *(lambda *a, lv=lv: _block(*a, lv) for lv in (2, 1, 0))):
+        p = _params(kind)
+        _attach(p, written, False)
+        xx = x.clone().requires_grad_()
+        y = run(kind, xx, cos, sin, SeqInfo.from_list(cu, DEV), p)
+        y.backward(dy)
+        got.append({"y": y.detach(), "x": xx.grad, **{n: t.main_grad for n, t in p.items() if t is not None}})
+    assert nv.get_error()[0] == 0
+    assert torch.equal(got[0]["y"], got[1]["y"])
+    for n, want in got[0].items():
+        assert torch.equal(got[1][n], got[2][n]) and torch.equal(got[1][n], got[3][n]), n
+        # one more rounding to bf16 where a residual's gradient is added (2^-9), through four products
+        assert ((got[1][n].float() - want.float()).norm() / want.float().norm()).item() < 8e-3, n
+
+
+@pytest.mark.parametrize("views", [False, True])
+@pytest.mark.parametrize("written", [False, True])
+@pytest.mark.parametrize("kind", ["vision", "text"])
+def test_no_rows(kind, written, views):
+    from multimodal_training_b200.ops.attention import SeqInfo
+    x, dy, cos, sin = _inputs(kind, 0)
+    p = _params(kind)
+    if views:
+        _attach(p, written, False)
+    before = {n: t.main_grad.clone() for n, t in p.items() if t is not None and views}
+    for level in (2, 1, 0):
+        xx = x.clone().requires_grad_()
+        y = _block(kind, xx, cos, sin, SeqInfo.from_list([0, 0], DEV), p, level)
+        y.backward(dy)
+        assert y.shape == x.shape and xx.grad.shape == x.shape
+    for n, t in p.items():
+        if t is not None and views:
+            assert t.grad_written and torch.equal(t.main_grad, before[n] if written else torch.zeros_like(t)), n
+        elif t is not None:
+            assert not t.grad.any()

@@ -61,12 +61,13 @@ def test_shapes_that_do_not_fill_the_gpu(M, N, K):
     assert _close(F.gemm(a, b), A.double() @ B.double().t(), K)
 
 
+@pytest.mark.parametrize("layout", ["kk", "k_mn", "mn_mn"])
 @pytest.mark.parametrize("bn", [64, 128, 192, 256])
-def test_one_tile_per_cta_has_the_bits_of_the_persistent_kernel(bn):
+def test_one_tile_per_cta_has_the_bits_of_the_persistent_kernel(bn, layout):
     from multimodal_training_b200.ops import functional as F
     from multimodal_training_b200.ops import native as nv
     torch.manual_seed(bn)
-    A, B, kw, a, b = _operands(264, 328, 1000, "kk")
+    A, B, kw, a, b = _operands(264, 328, 1000, layout)
     bias, res = torch.randn(328, device="cuda").bfloat16(), torch.randn(264, 328, device="cuda").bfloat16()
     got = []
     try:
