@@ -276,7 +276,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_co
       __syncwarp();
     }
   } else {
-    // ------------------------------ softmax warps (8) + epilogue ------------------------------
+    // ------------------------------ softmax warps (16) + epilogue ------------------------------
     const int q4 = warp & 3;               // tensor-memory lane quadrant
     const int part = warp >> 2;            // which 16 of the 64 query columns
     const int row = q4 * 32 + lane;        // kv row of this thread inside the tile
@@ -689,7 +689,7 @@ extern "C" int mmt_attn_bwd(const void* qkv, const void* out, const void* dout, 
   const bool split = ws != nullptr && n_q > n_kv;
   p.ws_dk = split ? ws : nullptr;
   p.ws_dv = split ? ws + (long)n_q * T * dim : nullptr;
-  CUtensorMap tq64, tdo64;   // 64-row boxes for the second-generation kernels' query / KV blocks
+  CUtensorMap tq64, tdo64;   // 64-row boxes: the query blocks of dK/dV, the KV blocks of dQ
   r = mmt_make_tmap_2d(&tq64, qkv, width, (uint64_t)T, (uint64_t)ld, 64, 64);
   if (r) return 3000 + r;
   r = mmt_make_tmap_2d(&tdo64, dout, (uint64_t)n_q * dim, (uint64_t)T, (uint64_t)n_q * dim, 64, 64);

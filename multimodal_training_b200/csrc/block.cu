@@ -1,6 +1,6 @@
 // One transformer block per call: the host side of ops/blocks.py in native code.
 //
-// A block is 9 launches forward and up to 26 backward.  Issued one by one from Python (a ctypes call with up to 21
+// A block is 9 launches forward and up to 21 backward.  Issued one by one from Python (a ctypes call with up to 21
 // arguments, an output allocation and several tensor lookups each) a launch costs 15-20 us of host time, which is more
 // than many of these kernels run: at 256 patches the vision encoder took 6.3 ms for 3.6 ms of device work.  Here a
 // block is one call with one array of addresses.

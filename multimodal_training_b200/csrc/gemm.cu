@@ -1627,11 +1627,6 @@ const MmtGemmComm* g_comm = nullptr;
 // Attach collective roles to the NEXT mmt_gemm_bf16 call of this thread of control (cleared by that call).
 extern "C" void mmt_gemm_set_comm(const MmtGemmComm* c) { g_comm = c; }
 
-// C = epilogue(alpha * A * B^T).  See the file header for layouts.
-//   a_mn / b_mn : 0 = K-major ([rows][K], ld = row stride), 1 = MN-major ([K][rows], ld = k-row stride)
-//   act         : 0 none, 1 GELU
-//   bn          : 0 = choose, else one of 64/128/192/256
-// Returns 0 or a CUDA / driver error code (negative: argument error).
 // A count that only the device knows (GemmParams::cnt) and, for a count of rows, the tile of this launch.
 struct GemmCount {
   const int* cnt;
@@ -1936,6 +1931,11 @@ static int gemm_call(const void* A, const void* B, void* C, const void* bias, co
   return rc;
 }
 
+// C = epilogue(alpha * A * B^T).  See the file header for layouts.
+//   a_mn / b_mn : 0 = K-major ([rows][K], ld = row stride), 1 = MN-major ([K][rows], ld = k-row stride)
+//   act         : 0 none, 1 GELU
+//   bn          : 0 = choose, else one of 64/128/192/256
+// Returns 0 or a CUDA / driver error code (negative: argument error).
 extern "C" int mmt_gemm_bf16(const void* A, const void* B, void* C, const void* bias, const void* residual, int M,
                              int N, int K, int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int act,
                              int accumulate, int out_f32, float alpha, int bn, void* stream) {

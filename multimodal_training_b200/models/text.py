@@ -154,7 +154,7 @@ class TextDecoder(nn.Module):
         """[T/tp, H] token shard -> final hidden token shard (before the last norm)."""
         x = x_shard
         # without tensor parallelism a layer has no communication inside and runs as one hand-written autograd
-        # node (ops/blocks.py); tensor-parallel layers, the CPU path and un-checkpointed runs use the per-op graph
+        # node (ops/blocks.py), with and without gradients; tensor-parallel layers and the CPU path use the per-op graph
         need = self.activation_bytes(bucket_tokens(x.shape[0]))       # token shards are equal on all TP ranks
         ckpt = decide_ckpt(self.ckpt, need, x.device, group=self.tp.group,
                            key=("text", id(self))) if torch.is_grad_enabled() else False
