@@ -1650,8 +1650,9 @@ static double wave_cost(int M, int N, long kb, int sms, int m, int width, bool s
 
 // The same for a product with collective roles, in units of one 256 x 256 x 64 step: waves x (k-blocks x c + e), with c and
 // e fitted (least squares over 200 sustained measurements on B200: the text shapes, the short-K vision shapes and the
-// tensor-parallel shards, all layouts).  Operand tiles that other ranks deliver are still fetched by a producer that one
-// lane runs, which is what these constants were taken with and those above were not.
+// tensor-parallel shards, all layouts) when one lane ran every producer.  Products that wait for other ranks' rows still
+// have such a producer; those that only store to other ranks share the plain loops, but not their stores.  Neither has been
+// measured with the constants above, so all of them keep these.
 static double collective_cost(int M, int N, long kb, int sms, int m, int width) {
   const long tiles = (long)((M + 128 * m - 1) / (128 * m)) * ((N + width - 1) / width);
   const double waves = (double)((tiles + sms - 1) / sms);
@@ -1674,9 +1675,9 @@ struct Tile {
 // 256 x 192 c 0.56 e 2.2).  c is close to what one SM's operand intake (about 110 GB/s) allows, so wide tiles win for
 // long K; e is the exposed epilogue of a 256-row tile, so 128-row tiles win for short K.  A last wave that is partly
 // empty has the L2 to itself and is up to a fifth faster.  What it mostly decides is how well the tile count fills
-// the 148 SMs.  (Constants from the time when issuing paced the 128-row tiles preferred 256 rows more often: 16384 x
-// 1280 x 1280 62.5 -> 50.6 us, 16384 x 1280 x 3840 135 -> 125, 6000 x 3840 x 1280 53.7 -> 49.1.)
-// Products with collective roles keep those earlier constants, see collective_cost.
+// the 148 SMs.  (The constants from the time when issuing paced the 128-row tiles, see collective_cost, prefer 256 rows
+// more often.  128 x 256 against 256 x 256 tiles today, us: 16384 x 3840 x 1280 123 and 138, 9000 x 6848 x 1280 120 and
+// 142, 16384 x 1280 x 3840 125 and 129; both models take 128 rows for 6000 x 3840 x 1280, 52 and 63.)
 // bn: 0 = choose, else the width asked for.
 static Tile choose_tile(int M, int N, long kb, int sms, int bn, bool collective) {
   auto cost = [&](int m, int width) {
